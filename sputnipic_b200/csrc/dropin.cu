@@ -152,7 +152,8 @@ int get_species(const struct particles *part, Species **out) {
     auto sp = std::make_unique<Species>();
     SPB_CUDA(cudaStreamCreateWithFlags(&sp->stream, cudaStreamNonBlocking));
     SPB_CUDA(cudaMalloc(&sp->d_err, sizeof(int)));
-    SPB_CUDA(cudaMemset(sp->d_err, 0, sizeof(int)));
+    SPB_CUDA(cudaMemsetAsync(sp->d_err, 0, sizeof(int), sp->stream));
+    SPB_CUDA(cudaStreamSynchronize(sp->stream));   // the pipeline's streams use it too
     it = st.species.emplace(part->x, std::move(sp)).first;
   }
   *out = it->second.get();

@@ -142,7 +142,8 @@ int create_from_coords(const std::vector<float> &xn, const std::vector<float> &y
   all.insert(all.end(), zn.begin(), zn.end());
   if (cudaMemcpy(c->d_nodes, all.data(), ncoord * sizeof(float), cudaMemcpyHostToDevice) !=
           cudaSuccess ||
-      cudaMemset(c->d_err, 0, sizeof(int)) != cudaSuccess)
+      cudaMemset(c->d_err, 0, sizeof(int)) != cudaSuccess ||
+      cudaStreamSynchronize(nullptr) != cudaSuccess)   // the caller's stream may not wait for it
     return cleanup(fail(SPB_ERR_CUDA, "spb_grid_create: upload failed"));
   GeomDev &g = c->geom;
   g.nxn = c->nxn;
@@ -324,7 +325,7 @@ extern "C" int spb_grid_check(spb_grid_ctx *c, void *stream) {
   int h = 0;
   SPB_CUDA(cudaMemcpy(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (h) {
-    SPB_CUDA(cudaMemset(c->d_err, 0, sizeof(int)));
+    SPB_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), (cudaStream_t)stream));
     return fail(SPB_ERR_OUT_OF_GRID,
                 "a particle cell index left the node array; the particle was clamped to the "
                 "edge cell");

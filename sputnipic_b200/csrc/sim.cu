@@ -2691,8 +2691,11 @@ extern "C" int spb_sim_create(const spb_sim_desc *d, spb_sim **out) {
     cudaGetLastError();
     return bail(fail(SPB_ERR_ALLOC, "spb_sim_create: device allocation failed"));
   }
-  if (cudaMemset(s->d_err, 0, sizeof(int)) != cudaSuccess ||
-      cudaMemset(s->fields8, 0, s->nodes * 8 * sizeof(float)) != cudaSuccess)
+  // zeroed on the pool's stream; load_species, moments and check order
+  // themselves after it (spb_sim::created), since the caller's stream may be
+  // one that the default stream does not block
+  cudaStream_t pst = pool_stream();
+  if (cudaMemsetAsync(s->d_err, 0, sizeof(int), pst) != cudaSuccess)
     return bail(fail(SPB_ERR_CUDA, "spb_sim_create: memset failed"));
   if (int rc = encode_field_map(s)) return bail(rc);
   s->sp.resize(d->ns);
@@ -2703,9 +2706,12 @@ extern "C" int spb_sim_create(const spb_sim_desc *d, spb_sim **out) {
       cudaGetLastError();
       return bail(fail(SPB_ERR_ALLOC, "spb_sim_create: device allocation failed"));
     }
-    if (cudaMemset(q.mom, 0, 10 * s->nodes * sizeof(double)) != cudaSuccess)
+    if (cudaMemsetAsync(q.mom, 0, 10 * s->nodes * sizeof(double), pst) != cudaSuccess)
       return bail(fail(SPB_ERR_CUDA, "spb_sim_create: memset failed"));
   }
+  if (cudaEventCreateWithFlags(&s->created, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventRecord(s->created, pst) != cudaSuccess)
+    return bail(fail(SPB_ERR_CUDA, "spb_sim_create: event failed"));
   *out = s;
   return SPB_OK;
 }
@@ -2849,6 +2855,7 @@ void spb::sim_free(spb_sim *s, bool sync) {
   if (s->gstream) cudaStreamDestroy(s->gstream);
   for (cudaEvent_t e : s->gev)
     if (e) cudaEventDestroy(e);
+  if (s->created) cudaEventDestroy(s->created);
   drain(s, nullptr, nullptr, nullptr, nullptr, nullptr);
   if (sync) cudaDeviceSynchronize();   // no queued work may still read the memory returned below
   for (auto &q : s->sp) {
@@ -2941,6 +2948,7 @@ extern "C" int spb_sim_load_species(spb_sim *s, int species, const float *x, con
   if (n >= (1L << 31) - 256)
     return fail(SPB_ERR_UNSUPPORTED, "spb_sim_load_species: at most 2^31 - 256 particles");
   cudaStream_t st = (cudaStream_t)stream;
+  SPB_CUDA(cudaStreamWaitEvent(st, s->created, 0));
   const float *src[7] = {x, y, z, u, v, w, q};
   Flat f;
   if (!on_device && n > 0) {
@@ -3050,6 +3058,7 @@ extern "C" int spb_sim_moments(spb_sim *s, int species, double *out, int on_devi
                                void *stream) {
   if (!s || !out || species < 0 || species >= (int)s->sp.size())
     return fail(SPB_ERR_INVALID, "spb_sim_moments: bad arguments");
+  if (!s->cycles_run) SPB_CUDA(cudaStreamWaitEvent((cudaStream_t)stream, s->created, 0));
   SPB_CUDA(cudaMemcpyAsync(out, s->sp[species].mom, 10 * s->nodes * sizeof(double),
                            on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                            (cudaStream_t)stream));
@@ -3128,9 +3137,10 @@ int sim_status(int h) {
 
 extern "C" int spb_sim_check(spb_sim *s, void *stream) {
   if (!s) return fail(SPB_ERR_INVALID, "spb_sim_check: null simulation");
+  SPB_CUDA(cudaEventSynchronize(s->created));
   SPB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
   int h = 0;
   SPB_CUDA(cudaMemcpy(&h, s->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (h) SPB_CUDA(cudaMemset(s->d_err, 0, sizeof(int)));
+  if (h) SPB_CUDA(cudaMemsetAsync(s->d_err, 0, sizeof(int), (cudaStream_t)stream));
   return spb::sim_status(h);
 }

@@ -72,6 +72,7 @@ struct spb_sim {
   int *fused_done = nullptr;      // fused cycle: [tiles] pushed flags + 2 barrier counters
   CUtensorMap fmap{};
   bool fields_set = false;
+  cudaEvent_t created = nullptr;  // the zeroing queued at creation is done
   int cycles_since_check = 0;
   // CUDA graphs of one cycle's launches, keyed by the species' buffer parities;
   // captured and replayed on gstream, ordered after the caller's stream

@@ -1,0 +1,43 @@
+"""Creating a simulation zeroes device memory; that zeroing has to come before what the caller
+queues next, also on a stream that the default stream does not block, and also while the default
+stream is busy. (Serving jobs admitted while others ran lost parts of their fields to it.)"""
+import pytest
+
+from sputnipic_b200 import workload as W
+
+pytestmark = pytest.mark.gpu
+
+
+def test_zeroing_comes_before_the_callers_stream(cuda):
+    torch = cuda
+    from sputnipic_b200 import device
+    from sputnipic_b200.sim import Simulation
+
+    wl = W.small_gem(nxc=16, nyc=8, nzc=8, E_amp=1e-3, species=W.gem_species((8, 8, 8, 8)))
+    fields = device.gen_fields(wl)
+    parts = [device.gen_particles(wl, s) for s in range(2)]
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+
+    def moments(busy):
+        if busy:
+            torch.cuda._sleep(200_000_000)   # about 0.1 s of the default stream
+        sim = Simulation(wl, species=[0, 1])
+        sim.set_fields(fields, stream=st)
+        for s, p in enumerate(parts):
+            sim.load_species(s, p, stream=st)
+        sim.cycle(1, stream=st)
+        st.synchronize()
+        torch.cuda.synchronize()   # whatever the creation left on the default stream
+        sim.cycle(1, stream=st)    # and what it left of the fields
+        assert sim.check(st) == 0
+        out = [sim.moments(s, stream=st) for s in range(2)]
+        st.synchronize()
+        sim.close()
+        return out
+
+    idle = moments(False)
+    for a, b in zip(idle, moments(True)):
+        assert float(a.norm()) > 0
+        # the same particles' FP32 cell sums in any order (the bar of the precision form)
+        assert float((a - b).norm() / a.norm()) <= 1e-5
