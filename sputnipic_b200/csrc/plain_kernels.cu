@@ -16,6 +16,7 @@
 // SoA streams through once (coalesced 4-byte loads per array per warp), the
 // 8-node gathers hit the packed fields, which stay L2-resident (14 MB at
 // 128x64x64 cells).
+#include "bc_fold.cuh"
 #include "grid_ctx.h"
 #include "warp_sum.cuh"
 
@@ -907,10 +908,6 @@ __global__ void __launch_bounds__(TPB) k_plain_mover_interp(
   if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
 }
 
-// applyBCids (src/BC.cpp:362-615), one launch per step so the axis order of
-// the reference holds: periodic folds X, Y, Z, then non-periodic doubling X,
-// Y, Z. Thread t handles one (row, col) pair of the boundary planes of all
-// ten moments.
 // sumOverSpecies (src/InterpDensNet.cpp:120-146) on the device: net moment m
 // of node i = the species' values added in species order, from zero, as the
 // reference's loop does (so the float sums are bit-identical).
@@ -944,45 +941,11 @@ __global__ void __launch_bounds__(TPB) k_fold_acc(const float4 *__restrict__ acc
   }
 }
 
-__global__ void __launch_bounds__(TPB) k_bc_fold(Moments10 M, int nxn, int nyn, int nzn,
-                                                 int axis, int periodic) {
-  int n1, n2;
-  if (axis == 0) {
-    n1 = nyn - 2;
-    n2 = nzn - 2;
-  } else if (axis == 1) {
-    n1 = nxn - 2;
-    n2 = nzn - 2;
-  } else {
-    n1 = nxn - 2;
-    n2 = nyn - 2;
-  }
+// applyBCids on the ten moments (blockIdx.y), see bc_fold.cuh.
+__global__ void __launch_bounds__(TPB) k_bc_fold(const __grid_constant__ Moments10 M,
+                                                 FoldGroups g) {
   const long t = blockIdx.x * (long)TPB + threadIdx.x;
-  if (t >= (long)n1 * n2) return;
-  const int r = 1 + (int)(t / n2), s = 1 + (int)(t % n2);
-  long lo, hi;
-  if (axis == 0) {
-    lo = ((long)1 * nyn + r) * nzn + s;
-    hi = ((long)(nxn - 2) * nyn + r) * nzn + s;
-  } else if (axis == 1) {
-    lo = ((long)r * nyn + 1) * nzn + s;
-    hi = ((long)r * nyn + (nyn - 2)) * nzn + s;
-  } else {
-    lo = ((long)r * nyn + s) * nzn + 1;
-    hi = ((long)r * nyn + s) * nzn + (nzn - 2);
-  }
-#pragma unroll
-  for (int m = 0; m < 10; ++m) {
-    float *a = M.m[m];
-    if (periodic) {
-      const float sum = a[lo] + a[hi];
-      a[lo] = sum;
-      a[hi] = sum;
-    } else {
-      a[lo] *= 2.0f;
-      a[hi] *= 2.0f;
-    }
-  }
+  if (t < g.fx + g.fy + g.fz) fold_group(g, M.m[blockIdx.y], t);
 }
 
 inline unsigned blocks_for(long n) { return (unsigned)ceil_div(n, TPB); }
@@ -1203,18 +1166,11 @@ int launch_apply_bc_ids(int nxn, int nyn, int nzn, const int periodic[3],
                         float *const mom[10], cudaStream_t s, long *launches) {
   Moments10 M;
   for (int m = 0; m < 10; ++m) M.m[m] = mom[m];
-  const long plane[3] = {(long)(nyn - 2) * (nzn - 2), (long)(nxn - 2) * (nzn - 2),
-                         (long)(nxn - 2) * (nyn - 2)};
-  // periodic folds in axis order, then the doubling of non-periodic axes
-  for (int pass = 0; pass < 2; ++pass)
-    for (int axis = 0; axis < 3; ++axis) {
-      const bool fold = periodic[axis] != 0;
-      if (fold != (pass == 0)) continue;
-      k_bc_fold<<<blocks_for(plane[axis]), TPB, 0, s>>>(M, nxn, nyn, nzn, axis, fold ? 1 : 0);
-      SPB_CUDA(cudaGetLastError());
-      g_launches++;
-      if (launches) ++*launches;
-    }
+  const FoldGroups g = fold_groups(nxn, nyn, nzn, periodic);
+  k_bc_fold<<<dim3(blocks_for(g.fx + g.fy + g.fz), 10), TPB, 0, s>>>(M, g);
+  SPB_CUDA(cudaGetLastError());
+  g_launches++;
+  if (launches) ++*launches;
   return SPB_OK;
 }
 

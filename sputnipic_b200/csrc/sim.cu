@@ -28,6 +28,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "bc_fold.cuh"
 #include "grid_ctx.h"
 #include "kernels.h"
 #include "sim_host.h"
@@ -1884,46 +1885,10 @@ __global__ void k_pack_fields8(const float *__restrict__ ex, const float *__rest
   }
 }
 
-// applyBCids (src/BC.cpp:362-615) on FP64 moments: periodic folds X, Y, Z,
-// then the doubling of non-periodic axes; one launch per step.
-__global__ void k_bc_fold64(double *mom, int nxn, int nyn, int nzn, int axis, int periodic) {
-  int n1, n2;
-  if (axis == 0) {
-    n1 = nyn - 2;
-    n2 = nzn - 2;
-  } else if (axis == 1) {
-    n1 = nxn - 2;
-    n2 = nzn - 2;
-  } else {
-    n1 = nxn - 2;
-    n2 = nyn - 2;
-  }
-  const long nodes = (long)nxn * nyn * nzn;
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= (long)n1 * n2) return;
-  const int r = 1 + (int)(t / n2), s = 1 + (int)(t % n2);
-  long lo, hi;
-  if (axis == 0) {
-    lo = ((long)1 * nyn + r) * nzn + s;
-    hi = ((long)(nxn - 2) * nyn + r) * nzn + s;
-  } else if (axis == 1) {
-    lo = ((long)r * nyn + 1) * nzn + s;
-    hi = ((long)r * nyn + (nyn - 2)) * nzn + s;
-  } else {
-    lo = ((long)r * nyn + s) * nzn + 1;
-    hi = ((long)r * nyn + s) * nzn + (nzn - 2);
-  }
-  for (int m = 0; m < 10; ++m) {
-    double *a = mom + m * nodes;
-    if (periodic) {
-      const double sum = a[lo] + a[hi];
-      a[lo] = sum;
-      a[hi] = sum;
-    } else {
-      a[lo] *= 2.0;
-      a[hi] *= 2.0;
-    }
-  }
+// applyBCids on a species' ten FP64 moments (blockIdx.y), see bc_fold.cuh.
+__global__ void __launch_bounds__(256) k_bc_fold64(double *mom, long nodes, FoldGroups g) {
+  const long t = blockIdx.x * 256L + threadIdx.x;
+  if (t < g.fx + g.fy + g.fz) fold_group(g, mom + blockIdx.y * nodes, t);
 }
 
 int blocks_for(long n, int tpb) {
@@ -3077,18 +3042,12 @@ extern "C" int spb_sim_apply_bc_ids(spb_sim *s, int species, void *stream) {
   if (!s || species < 0 || species >= (int)s->sp.size())
     return fail(SPB_ERR_INVALID, "spb_sim_apply_bc_ids: bad arguments");
   cudaStream_t st = (cudaStream_t)stream;
-  const long plane[3] = {(long)(s->nyn - 2) * (s->nzn - 2), (long)(s->nxn - 2) * (s->nzn - 2),
-                         (long)(s->nxn - 2) * (s->nyn - 2)};
-  for (int pass = 0; pass < 2; ++pass)
-    for (int axis = 0; axis < 3; ++axis) {
-      const bool fold = s->d.periodic[axis] != 0;
-      if (fold != (pass == 0)) continue;
-      k_bc_fold64<<<(unsigned)ceil_div(plane[axis], 256), 256, 0, st>>>(
-          s->sp[species].mom, s->nxn, s->nyn, s->nzn, axis, fold ? 1 : 0);
-      SPB_CUDA(cudaGetLastError());
-      g_launches++;
-      s->launches++;
-    }
+  const FoldGroups g = fold_groups(s->nxn, s->nyn, s->nzn, s->d.periodic);
+  k_bc_fold64<<<dim3((unsigned)ceil_div(g.fx + g.fy + g.fz, 256), 10), 256, 0, st>>>(
+      s->sp[species].mom, s->nodes, g);
+  SPB_CUDA(cudaGetLastError());
+  g_launches++;
+  s->launches++;
   return SPB_OK;
 }
 
