@@ -33,7 +33,7 @@
 #include "kernels.h"
 #include "sim_host.h"
 #include "sim_kernels.cuh"
-#include "warp_sum.cuh"
+#include "cell_deposit.cuh"
 
 namespace spb {
 namespace {
@@ -398,43 +398,6 @@ __device__ __forceinline__ void push(const CycleParams &P, const float *__restri
   }
 }
 
-// Deposit terms of one particle added to 40 packed accumulators:
-// acc[node*5 + k] += W_node * (mf[k], mf[k+5]) with the moment factors
-// mf = 1, u, v, w, uu | uv, uw, vv, vw, ww, i.e. the pairs (1,uv) (u,uw)
-// (v,vv) (w,vw) (uu,ww), in the reference order rhon, Jx, Jy, Jz, pxx | pxy,
-// pxz, pyy, pyz, pzz (src/Mover.cpp:466-570); node = a*4 + b*2 + c with
-// a/b/c = 1 the upper node on that axis, XOR-permuted by bits 4/3/2 of
-// `perm` (the lane for warp_sum80, 0 for the plain order). q is folded into
-// the x weights; q = 0 adds nothing.
-__device__ __forceinline__ void add_terms(float2 (&acc)[40], float q, float ox, float oy, float oz,
-                                          float u, float v, float w, int perm) {
-  const bool px = perm & 16, py = perm & 8, pz = perm & 4;
-  const float lox = 1.0f - ox, loy = 1.0f - oy, loz = 1.0f - oz;
-  const float wx0 = q * (px ? ox : lox), wx1 = q * (px ? lox : ox);
-  const float wy0 = py ? oy : loy, wy1 = py ? loy : oy;
-  const float wz0 = pz ? oz : loz, wz1 = pz ? loz : oz;
-  const float2 mf[5] = {make_float2(1.0f, u * v), make_float2(u, u * w), make_float2(v, v * v),
-                        make_float2(w, v * w), make_float2(u * u, w * w)};
-  const float wxy[4] = {wx0 * wy0, wx0 * wy1, wx1 * wy0, wx1 * wy1};
-#pragma unroll
-  for (int ab = 0; ab < 4; ++ab) {
-    const float W0 = wxy[ab] * wz0, W1 = wxy[ab] * wz1;
-    const float2 W02 = make_float2(W0, W0), W12 = make_float2(W1, W1);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      acc[(ab * 2 + 0) * 5 + k] = __ffma2_rn(W02, mf[k], acc[(ab * 2 + 0) * 5 + k]);
-      acc[(ab * 2 + 1) * 5 + k] = __ffma2_rn(W12, mf[k], acc[(ab * 2 + 1) * 5 + k]);
-    }
-  }
-}
-
-// One 32-byte record store (one 256-bit access; p 32-byte aligned).
-__device__ __forceinline__ void st_rec(float4 *p, float4 a, float4 b) {
-  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x),
-               "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
-               : "memory");
-}
-
 // Stores one pushed record in slot `slot` of the bucket [dbase, dend) of cell
 // `key`, or appends it to the overflow list when the bucket is full. Returns
 // 1 if the overflow list was full too (the particle is lost; reported).
@@ -510,7 +473,25 @@ struct JobTable {
   int njobs, total_tiles;
   const int *tile_base;          // [njobs + 1] first launch-wide tile of each job
   const CycleParams *params;     // [njobs]
+  int split;                     // work items are (species, tile) pairs, not tiles (one
+                                 // simulation too): tile_base and total_tiles count them
 };
+
+// Work item `local` of job P: its tile and species [s0, s1). Split items are
+// numbered species by species, so that with fewer tiles than CTAs no CTA gets
+// two items of one species before every CTA has one.
+__device__ __forceinline__ void work_item(const CycleParams &P, int split, int local, int &tile,
+                                          int &s0, int &s1) {
+  tile = local;
+  s0 = 0;
+  s1 = P.ns;
+  if (split) {
+    const int nt = P.ntx * P.nty * P.ntz;
+    s0 = local / nt;
+    s1 = s0 + 1;
+    tile = local - s0 * nt;
+  }
+}
 
 // The jobs' field maps travel as a kernel parameter, like the single job's.
 struct JobMaps {
@@ -554,7 +535,7 @@ struct PushWarp {
   int bad = 0, lost = 0;
 };
 
-// All species of one tile (tile-local index `tile` of the job P) on the
+// Species [s0, s1) of one tile (tile-local index `tile` of the job P) on the
 // staged fields sF. All threads call.
 //
 // Each warp owns NC cells of the tile (tile-local warp + j * NW) and pushes
@@ -571,15 +552,15 @@ __device__ __forceinline__ bool far_axis(int d, int n, int periodic) {
 }
 
 template <int TX, int TY, int TZ, int RH, bool FUSED = false>
-__device__ __forceinline__ void push_tile(const CycleParams &P, int tile, const float *sF,
-                                          PushWarp &W) {
+__device__ __forceinline__ void push_tile(const CycleParams &P, int tile, int s0, int s1,
+                                          const float *sF, PushWarp &W) {
   using T = Tile<TX, TY, TZ>;
   constexpr int NC = T::TC / SIM_NW;   // cells per warp and tile
   static_assert(RH % 32 == 0, "slots must not straddle ring halves");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tz = tile % P.ntz, ty = (tile / P.ntz) % P.nty, tx = tile / (P.ntz * P.nty);
   const int c0x = tx * TX, c0y = ty * TY, c0z = tz * TZ;
-  for (int s = 0; s < P.ns; ++s) {
+  for (int s = s0; s < s1; ++s) {
     const SpeciesDev &S = P.sp[s];
     // lane j < NC: bucket start and particle count of the warp's j-th cell,
     // and cp = the cell's first index in the warp's stream
@@ -783,20 +764,21 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
   }
   __syncthreads();
 
-  const int ntiles = MULTI ? J.total_tiles : P1.ntx * P1.nty * P1.ntz;
-  auto locate_tile = [&](int t, int &job, int &local) {
+  const int ntiles = MULTI ? J.total_tiles
+                           : P1.ntx * P1.nty * P1.ntz * (J.split ? P1.ns : 1);
+  auto locate_tile = [&](int t, int &job, int &local, int &s0, int &s1) {
     if constexpr (MULTI) {
       job = job_of(J, t);
-      local = t - J.tile_base[job];
+      work_item(J.params[job], J.split, t - J.tile_base[job], local, s0, s1);
     } else {
       job = 0;
-      local = t;
+      work_item(P1, J.split, t, local, s0, s1);
     }
   };
   const unsigned box_bytes = (unsigned)(T::BN * 8 * sizeof(float));
   auto issue = [&](int t, int stage) {   // thread 0
-    int job, local;
-    locate_tile(t, job, local);
+    int job, local, s0, s1;
+    locate_tile(t, job, local, s0, s1);
     const int nty = MULTI ? J.params[job].nty : P1.nty;
     const int ntz = MULTI ? J.params[job].ntz : P1.ntz;
     const CUtensorMap *map;
@@ -827,17 +809,17 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
       return;
     }
     const float *sF = sF0 + stage * T::SF;
-    int job, local;
-    locate_tile(tile, job, local);
+    int job, local, s0, s1;
+    locate_tile(tile, job, local, s0, s1);
     if constexpr (MULTI) {
       if (job != cur_job) {
         load_params(sP, J.params + job);
         cur_job = job;
       }
-      push_tile<TX, TY, TZ, RH>(*sP, local, sF, W);
+      push_tile<TX, TY, TZ, RH>(*sP, local, s0, s1, sF, W);
       report(*sP, W);
     } else {
-      push_tile<TX, TY, TZ, RH>(P1, local, sF, W);
+      push_tile<TX, TY, TZ, RH>(P1, local, s0, s1, sF, W);
     }
     // every warp is done with this field stage (and the staged parameters)
     // before they are refilled
@@ -962,15 +944,6 @@ __host__ __device__ constexpr int dep_tpb() {
   return ((TX * TY * TZ + 31) / 32) * 32;
 }
 
-// Read-only 32-byte load of one particle record (one 256-bit access) that asks
-// L2 to fetch the surrounding 256 bytes: a lane walking its cell's bucket then
-// finds the next records in L2.
-__device__ __forceinline__ void ld_rec(const float4 *p, float4 &a, float4 &b) {
-  asm("ld.global.nc.L2::256B.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-      : "l"(p));
-}
-
 // The same through L2 only (coherent with records written by other CTAs of
 // the same launch, which the fused cycle deposits).
 __device__ __forceinline__ void ld_rec_cg(const float4 *p, float4 &a, float4 &b) {
@@ -987,33 +960,29 @@ __device__ __forceinline__ void ld_record(const float4 *p, float4 &a, float4 &b)
     ld_rec(p, a, b);
 }
 
-// Per-warp quota of the deposit (all 32 lanes call with their cell's count):
-// lanes sum at most Q particles of their own cell, one particle per lane per
-// step; the excess of the cells above Q is summed by the whole warp, 32
-// particles per step plus one warp reduction per cell. Q minimises the
-// estimated issue slots, 60 per lane step and 65 per warp step + 160 per
-// excess cell, over the candidates Q = one of the lanes' counts; a warp whose
-// largest count is at most 1.25 x its mean keeps Q = its largest count.
-__device__ __forceinline__ int deposit_quota(int cnt) {
-  const int mx = __reduce_max_sync(FULL, cnt);
-  if (mx > (1 << 24)) return mx;   // keeps the cost sums below 2^32
-  const int sum = __reduce_add_sync(FULL, cnt);
-  if ((long long)mx * 32 * 4 <= (long long)sum * 5) return mx;   // max <= 1.25 x mean
-  unsigned cost = 60u * (unsigned)cnt;
-#pragma unroll 4
-  for (int i = 0; i < 32; ++i) {
-    const int c = __shfl_sync(FULL, cnt, i);
-    if (c > cnt) cost += 65u * (unsigned)((c - cnt + 31) >> 5) + 160u;
-  }
-  const unsigned lane = threadIdx.x & 31;
-  const unsigned best = __reduce_min_sync(FULL, (min(cost, (1u << 26) - 1) << 5) | lane);
-  return __shfl_sync(FULL, cnt, (int)(best & 31u));
+// Adds a tile's node sums (scale: 1, or invVOL) into a species' moments, one
+// FP64 atomic per node and moment.
+template <int TX, int TY, int TZ, int NT, typename T>
+__device__ __forceinline__ void add_node_sums(const CycleParams &P, double *__restrict__ mom,
+                                              const typename PairOf<T>::type *sCell, int c0x,
+                                              int c0y, int c0z, double scale) {
+  const long nodes = (long)P.nxn * P.nyn * P.nzn;
+  node_sums<TX, TY, TZ, NT, T>(
+      sCell, [&](int bx, int by, int bz, const typename PairOf<T>::type(&sum)[5]) {
+        double *to =
+            mom + ((long)(c0x + bx + 1) * P.nyn + (c0y + by + 1)) * P.nzn + (c0z + bz + 1);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+          if (sum[k].x != (T)0) atomicAdd(to + k * nodes, (double)sum[k].x * scale);
+          if (sum[k].y != (T)0) atomicAdd(to + (k + 5) * nodes, (double)sum[k].y * scale);
+        }
+      });
 }
 
-// All species of one tile (tile-local index `tile` of job P). Thread t owns
+// Species [s0, s1) of one tile (tile-local index `tile` of job P). Thread t owns
 // cell t of the tile: it walks the cell's bucket, accumulating the 80 terms
 // of every particle in packed FP32 registers (no cross-lane reduction), and
-// stores the cell's totals in shared memory, term-major (sCell[j * TC + t]).
+// stores the cell's totals in shared memory (see PairOf).
 // Each node of the tile then adds up the totals of its (up to 8) cells in the
 // tile and one FP64 atomic per node and moment adds the sum into the moments.
 // All threads call.
@@ -1021,17 +990,15 @@ __device__ __forceinline__ int deposit_quota(int cnt) {
 // counters and records (the fused cycle, where other CTAs of the launch wrote
 // them).
 template <int TX, int TY, int TZ, int NT = dep_tpb<TX, TY, TZ>(), bool COH = false>
-__device__ __forceinline__ void deposit_tile(const CycleParams &P, int tile, float *sCell) {
-  using T = Tile<TX, TY, TZ>;
-  constexpr int NX = TX + 1, NY = TY + 1, NZ = TZ + 1, NB = NX * NY * NZ;
-  constexpr int TC = T::TC;
+__device__ __forceinline__ void deposit_tile(const CycleParams &P, int tile, int s0, int s1,
+                                             float2 *sCell) {
+  constexpr int TC = Tile<TX, TY, TZ>::TC;
   static_assert(NT >= TC && NT % 32 == 0, "one thread per cell, whole warps");
   const int tid = threadIdx.x;
   const bool own = tid < TC;
-  const long nodes = (long)P.nxn * P.nyn * P.nzn;
   const int tz = tile % P.ntz, ty = (tile / P.ntz) % P.nty, tx = tile / (P.ntz * P.nty);
   const int c0x = tx * TX, c0y = ty * TY, c0z = tz * TZ;
-  for (int s = 0; s < P.ns; ++s) {
+  for (int s = s0; s < s1; ++s) {
     const SpeciesDev &S = P.sp[s];
     const float4 *rec = S.rout;
     int cnt = 0;
@@ -1058,7 +1025,8 @@ __device__ __forceinline__ void deposit_tile(const CycleParams &P, int tile, flo
       // count add zero terms
       float4 na = a1, nb = b1;
       if (k + 2 < n1) ld_record<COH>(rec + 2 * (k + 2), na, nb);
-      add_terms(acc, k < n1 ? a.w : 0.0f, a.x, a.y, a.z, b.x, b.y, b.z, 0);
+      add_terms(acc, k < n1 ? a.w : 0.0f, 1.0f - a.x, a.x, 1.0f - a.y, a.y, 1.0f - a.z, a.z, b.x,
+                b.y, b.z, 0);
       a = a1;
       b = b1;
       a1 = na;
@@ -1067,9 +1035,7 @@ __device__ __forceinline__ void deposit_tile(const CycleParams &P, int tile, flo
     if (own) {
 #pragma unroll
       for (int i = 0; i < 40; ++i) {
-        const int node = i / 5, k = i % 5;
-        sCell[(node * 10 + k) * TC + tid] = acc[i].x;
-        sCell[(node * 10 + k + 5) * TC + tid] = acc[i].y;
+        sCell[i * TC + tid] = acc[i];   // i = corner * 5 + k
       }
     }
     // the cells above the quota: particles Q.. of each, one per lane, summed
@@ -1093,36 +1059,19 @@ __device__ __forceinline__ void deposit_tile(const CycleParams &P, int tile, flo
           const int i = o + lane;
           float4 ha = make_float4(0.f, 0.f, 0.f, 0.f), hb = ha;
           if (i < hc) ld_record<COH>(hrec + 2 * i, ha, hb);
-          add_terms(acc, i < hc ? ha.w : 0.0f, ha.x, ha.y, ha.z, hb.x, hb.y, hb.z, lane);
+          add_terms(acc, i < hc ? ha.w : 0.0f, 1.0f - ha.x, ha.x, 1.0f - ha.y, ha.y, 1.0f - ha.z,
+                    ha.z, hb.x, hb.y, hb.z, lane);
         }
         float r[5];
         warp_sum80(acc, r, lane);
-        float *dst = sCell + (corner * 10 + mbase) * TC + wbase + hl;
+        float2 *dst = sCell + corner * 5 * TC + wbase + hl;
 #pragma unroll
         for (int k = 0; k < 5; ++k)
-          if (k >= lo && k < hi) dst[k * TC] += r[k];
+          if (k >= lo && k < hi) (mbase ? dst[k * TC].y : dst[k * TC].x) += r[k];
       }
     }
     __syncthreads();
-    for (int idx = tid; idx < 10 * NB; idx += NT) {
-      const int m = idx / NB, nb = idx % NB;
-      const int bz = nb % NZ, by = (nb / NZ) % NY, bx = nb / (NZ * NY);
-      float sum = 0.0f;
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int lx = bx - a, ly = by - b, lz = bz - c;
-            if (lx >= 0 && lx < TX && ly >= 0 && ly < TY && lz >= 0 && lz < TZ)
-              sum += sCell[((a * 4 + b * 2 + c) * 10 + m) * TC + (lx * TY + ly) * TZ + lz];
-          }
-      if (sum != 0.0f) {
-        const long g = ((long)(c0x + bx + 1) * P.nyn + (c0y + by + 1)) * P.nzn + (c0z + bz + 1);
-        atomicAdd(S.mom + m * nodes + g, (double)sum * P.scale);
-      }
-    }
+    add_node_sums<TX, TY, TZ, NT, float>(P, S.mom, sCell, c0x, c0y, c0z, P.scale);
     __syncthreads();
   }
 }
@@ -1134,17 +1083,14 @@ __device__ __forceinline__ void deposit_tile(const CycleParams &P, int tile, flo
 // its (up to 8) cells' sums and issues one FP64 atomic per moment, all exact.
 // The moments stay unscaled until k_scale_moments. All threads call.
 template <int TX, int TY, int TZ>
-__device__ __forceinline__ void deposit_tile_exact(const CycleParams &P, int tile, double *sCell,
-                                                   int &inexact) {
-  using T = Tile<TX, TY, TZ>;
-  constexpr int NX = TX + 1, NY = TY + 1, NZ = TZ + 1, NB = NX * NY * NZ;
-  constexpr int TC = T::TC, NT = dep_tpb<TX, TY, TZ>();
+__device__ __forceinline__ void deposit_tile_exact(const CycleParams &P, int tile, int s0, int s1,
+                                                   double2 *sCell, int &inexact) {
+  constexpr int TC = Tile<TX, TY, TZ>::TC, NT = dep_tpb<TX, TY, TZ>();
   const int tid = threadIdx.x;
   const bool own = tid < TC;
-  const long nodes = (long)P.nxn * P.nyn * P.nzn;
   const int tz = tile % P.ntz, ty = (tile / P.ntz) % P.nty, tx = tile / (P.ntz * P.nty);
   const int c0x = tx * TX, c0y = ty * TY, c0z = tz * TZ;
-  for (int s = 0; s < P.ns; ++s) {
+  for (int s = s0; s < s1; ++s) {
     const SpeciesDev &S = P.sp[s];
     const double M[3] = {exact_offset(S.quantum[0]), exact_offset(S.quantum[1]),
                          exact_offset(S.quantum[2])};
@@ -1182,32 +1128,15 @@ __device__ __forceinline__ void deposit_tile_exact(const CycleParams &P, int til
     if (own) {
 #pragma unroll
       for (int i = 0; i < 80; ++i) {
-        const int k = (i % 10) == 0 ? 0 : ((i % 10) < 4 ? 1 : 2);
+        const int m = i % 10, k = m == 0 ? 0 : (m < 4 ? 1 : 2);
         const double lo = 4503599627370496.0 * S.quantum[k];   // 2^52 Q; 2^53 Q above
         inexact |= (acc[i] < lo) | (acc[i] >= 2.0 * lo);
-        sCell[i * TC + tid] = (acc[i] - M[k]) + (double)cnt * 0.5 * S.quantum[k];
+        double2 &to = sCell[((i / 10) * 5 + m % 5) * TC + tid];
+        (m < 5 ? to.x : to.y) = (acc[i] - M[k]) + (double)cnt * 0.5 * S.quantum[k];
       }
     }
     __syncthreads();
-    for (int idx = tid; idx < 10 * NB; idx += NT) {
-      const int m = idx / NB, nb = idx % NB;
-      const int bz = nb % NZ, by = (nb / NZ) % NY, bx = nb / (NZ * NY);
-      double sum = 0.0;
-#pragma unroll
-      for (int a2 = 0; a2 < 2; ++a2)
-#pragma unroll
-        for (int b2 = 0; b2 < 2; ++b2)
-#pragma unroll
-          for (int c2 = 0; c2 < 2; ++c2) {
-            const int lx = bx - a2, ly = by - b2, lz = bz - c2;
-            if (lx >= 0 && lx < TX && ly >= 0 && ly < TY && lz >= 0 && lz < TZ)
-              sum += sCell[((a2 * 4 + b2 * 2 + c2) * 10 + m) * TC + (lx * TY + ly) * TZ + lz];
-          }
-      if (sum != 0.0) {
-        const long g = ((long)(c0x + bx + 1) * P.nyn + (c0y + by + 1)) * P.nzn + (c0z + bz + 1);
-        atomicAdd(S.mom + m * nodes + g, sum);
-      }
-    }
+    add_node_sums<TX, TY, TZ, NT, double>(P, S.mom, sCell, c0x, c0y, c0z, 1.0);
     __syncthreads();
   }
 }
@@ -1266,7 +1195,8 @@ __device__ __forceinline__ void deposit_overflow(const CycleParams &P) {
         float2 acc[40];
 #pragma unroll
         for (int j = 0; j < 40; ++j) acc[j] = make_float2(0.f, 0.f);
-        add_terms(acc, member ? a.w : 0.0f, a.x, a.y, a.z, b.x, b.y, b.z, lane);
+        add_terms(acc, member ? a.w : 0.0f, 1.0f - a.x, a.x, 1.0f - a.y, a.y, 1.0f - a.z, a.z, b.x,
+                  b.y, b.z, lane);
         float r[5];
         warp_sum80(acc, r, lane);
         int cx, cy, cz;
@@ -1297,18 +1227,21 @@ __global__ void __launch_bounds__(dep_tpb<TX, TY, TZ>(),
                                                ? 256 / dep_tpb<TX, TY, TZ>() : 1)
                                         : 512 / dep_tpb<TX, TY, TZ>())
     k_deposit(const __grid_constant__ CycleParams P1, const __grid_constant__ JobTable J) {
-  using T = Tile<TX, TY, TZ>;
   static_assert(!(MULTI && EXACT), "the deterministic deposit runs one simulation");
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  float *sCell = reinterpret_cast<float *>(smem_raw);   // 80 x TC (float, or double if EXACT)
-  CycleParams *sP =
-      reinterpret_cast<CycleParams *>(smem_raw + (size_t)T::TC * 80 * (EXACT ? 8 : 4));   // MULTI
-  const int ntiles = MULTI ? J.total_tiles : P1.ntx * P1.nty * P1.ntz;
-  int cur_job = -1;
+  float2 *sCell = reinterpret_cast<float2 *>(smem_raw);   // 40 x TC pairs (double2 if EXACT)
+  CycleParams *sP = reinterpret_cast<CycleParams *>(
+      smem_raw + (size_t)Tile<TX, TY, TZ>::TC * 80 * (EXACT ? 8 : 4));   // MULTI
+  const int ntiles = MULTI ? J.total_tiles
+                           : P1.ntx * P1.nty * P1.ntz * (J.split ? P1.ns : 1);
+  int cur_job = -1, local, s0, s1;
   if constexpr (EXACT) {
     int inexact = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-      deposit_tile_exact<TX, TY, TZ>(P1, tile, reinterpret_cast<double *>(smem_raw), inexact);
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+      work_item(P1, J.split, tile, local, s0, s1);
+      deposit_tile_exact<TX, TY, TZ>(P1, local, s0, s1, reinterpret_cast<double2 *>(smem_raw),
+                                     inexact);
+    }
     if (inexact) atomicOr(P1.err, ERRBIT_INEXACT);
     deposit_overflow<TX, TY, TZ, true>(P1);
   } else {
@@ -1320,9 +1253,11 @@ __global__ void __launch_bounds__(dep_tpb<TX, TY, TZ>(),
           load_params(sP, J.params + job);
           cur_job = job;
         }
-        deposit_tile<TX, TY, TZ>(*sP, tile - J.tile_base[job], sCell);
+        work_item(*sP, J.split, tile - J.tile_base[job], local, s0, s1);
+        deposit_tile<TX, TY, TZ>(*sP, local, s0, s1, sCell);
       } else {
-        deposit_tile<TX, TY, TZ>(P1, tile, sCell);
+        work_item(P1, J.split, tile, local, s0, s1);
+        deposit_tile<TX, TY, TZ>(P1, local, s0, s1, sCell);
       }
     }
     if constexpr (MULTI) {
@@ -1482,7 +1417,7 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
                                                fused_rec_bytes<TX, TY, TZ, MINB>());   // 2 + 2 NW
   // the deposit's per-cell sums reuse the record staging and ring (idle
   // between two tiles' pushes; the field stages stay untouched)
-  float *sCell = reinterpret_cast<float *>(sRec);
+  float2 *sCell = reinterpret_cast<float2 *>(sRec);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   PushWarp W;
@@ -1530,7 +1465,7 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
         return;
       }
       const int tile = tile_of_order(P, o);
-      push_tile<TX, TY, TZ, RH, true>(P, tile, sF0 + stage * T::SF, W);
+      push_tile<TX, TY, TZ, RH, true>(P, tile, 0, P.ns, sF0 + stage * T::SF, W);
       if (__syncthreads_or(W.dead)) {
         if (tid == 0) atomicOr(P.err, ERRBIT_TIMEOUT);
         for (int b = 0; b < 2; ++b)
@@ -1551,7 +1486,7 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
         if (o + G < ntiles) mbar_wait_bounded(bar + (it & 1), (it >> 1) & 1);
         return;
       }
-      deposit_tile<TX, TY, TZ, SIM_TPB, true>(P, tile, sCell);
+      deposit_tile<TX, TY, TZ, SIM_TPB, true>(P, tile, 0, P.ns, sCell);
       // the next tile's bulk copies overwrite the sums written here
       fence_proxy_async();
       __syncthreads();
@@ -2049,6 +1984,17 @@ CycleParams make_params(spb_sim *s) {
 
 namespace {
 
+// Whether the work items of a launch are (species, tile) pairs instead of
+// tiles that a CTA takes all species of: when there are fewer tiles than CTAs
+// fit on the device. A pair stages its tile's fields again (17 KB against the
+// 0.1 to 1 MB of records of 27 to 125 particles per cell), so there is nothing
+// to gain once every CTA has a tile. 32x16x16 cells, 27 per cell, 4 species
+// (64 tiles, 444 and 592 CTAs): push
+// 116 -> 46 us, deposit 57 -> 20 us (half of the latter from node_sums).
+int split_items(int ntiles, int ns, int max_ctas) {
+  return ns > 1 && ntiles < max_ctas ? 1 : 0;
+}
+
 // One cycle: zero the moments and the write-side counters, push, deposit.
 template <int TX, int TY, int TZ, int MINB>
 int launch_cycle_v(spb_sim *s, cudaStream_t st) {
@@ -2093,14 +2039,20 @@ int launch_cycle_v(spb_sim *s, cudaStream_t st) {
     docc[0] = std::max(docc[0], 1);
     docc[1] = std::max(docc[1], 1);
   }
-  const int pctas = std::min(ntiles, s->d.ctas > 0 ? s->d.ctas : pocc * num_sms());
-  const int dctas = std::min(ntiles, docc[exact ? 1 : 0] * num_sms());
+  // with fewer tiles than CTAs fit, the species of a tile go to different
+  // CTAs (split_items)
+  const int pmax = s->d.ctas > 0 ? s->d.ctas : pocc * num_sms();
+  const int dmax = docc[exact ? 1 : 0] * num_sms();
+  JobTable jp{}, jd{};
+  jp.split = split_items(ntiles, P.ns, pmax);
+  jd.split = split_items(ntiles, P.ns, dmax);
+  const int pctas = std::min(jp.split ? ntiles * P.ns : ntiles, pmax);
+  const int dctas = std::min(jd.split ? ntiles * P.ns : ntiles, dmax);
   EvCycle ev{record_event(s, st), nullptr, nullptr};
-  k_push<TX, TY, TZ, MINB, false><<<pctas, SIM_TPB, psm, st>>>(s->fmap, P, JobTable{},
-                                                                      NoMaps{});
+  k_push<TX, TY, TZ, MINB, false><<<pctas, SIM_TPB, psm, st>>>(s->fmap, P, jp, NoMaps{});
   SPB_CUDA(cudaGetLastError());
   ev.m = record_event(s, st);
-  kdep<<<dctas, dep_tpb<TX, TY, TZ>(), dsm, st>>>(P, JobTable{});
+  kdep<<<dctas, dep_tpb<TX, TY, TZ>(), dsm, st>>>(P, jd);
   SPB_CUDA(cudaGetLastError());
   if (exact) {
     k_scale_moments<<<2 * num_sms(), 256, 0, st>>>(P);
@@ -2480,11 +2432,16 @@ int launch_jobs_t(spb_sim *const *sims, int n, JobBuffers &B, cudaStream_t st) {
   if (n > SERVE_MAX_JOBS) return fail(SPB_ERR_CAPACITY, "at most 64 jobs per launch");
   if (int rc = ensure_job_buffers(B, n)) return rc;
   static JobMaps maps;   // 8 KB, passed by value as a kernel parameter
-  int total = 0;
+  int tiles = 0, total = 0, nsmax = 1;
+  for (int j = 0; j < n; ++j) {
+    tiles += sims[j]->nt[0] * sims[j]->nt[1] * sims[j]->nt[2];
+    nsmax = std::max(nsmax, (int)sims[j]->sp.size());
+  }
+  const int split = split_items(tiles, nsmax, std::min(pocc, docc) * num_sms());
   for (int j = 0; j < n; ++j) {
     spb_sim *s = sims[j];
     B.h_tile_base[j] = total;
-    total += s->nt[0] * s->nt[1] * s->nt[2];
+    total += s->nt[0] * s->nt[1] * s->nt[2] * (split ? (int)s->sp.size() : 1);
     B.h_params[j] = make_params(s);
     maps.m[j] = s->fmap;
   }
@@ -2494,7 +2451,7 @@ int launch_jobs_t(spb_sim *const *sims, int n, JobBuffers &B, cudaStream_t st) {
   SPB_CUDA(cudaMemcpyAsync(B.d_params, B.h_params, n * sizeof(CycleParams),
                            cudaMemcpyHostToDevice, st));
   SPB_CUDA(cudaEventRecord(B.ready, st));
-  const JobTable J{n, total, B.d_tile_base, B.d_params};
+  const JobTable J{n, total, B.d_tile_base, B.d_params, split};
   k_zero_jobs<<<2 * num_sms(), 256, 0, st>>>(J);
   SPB_CUDA(cudaGetLastError());
   const int pctas = std::min(total, pocc * num_sms());
