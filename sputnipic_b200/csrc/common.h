@@ -31,6 +31,12 @@ struct GeomDev {
   float invdx, invdy, invdz, invVOL;
   double Lx, Ly, Lz;
   const float *xn, *yn, *zn;  // node coordinates per axis (device)
+  const float2 *xp, *yp, *zp;  // (node i - 1, node i) pairs per axis (device), i >= 1
+  float Lfx, Lfy, Lfz;         // the largest floats not above Lx, Ly, Lz
+  float nxf, nyf, nzf;         // nxn - 2, nyn - 2, nzn - 2
+  // the domain starts at 0 on every axis and no axis has 2^22 nodes: cell
+  // indices can be formed in float (cell_index)
+  int float_cells;
 };
 
 // Time-step constants of mover_PC (src/Mover.cpp:11-12), already rounded
@@ -41,11 +47,13 @@ struct PushDev {
   int periodic[3];
 };
 
-// Packed node fields: one float4 (Ex, Ey, Ez, Bx) and one float2 (By, Bz)
-// per node, so a node's six components arrive in two loads.
+// Packed node fields: three float4 per node n of the row z = 0..nzn-1, each
+// component of node n beside that of node n - 1 (the node below it on z):
+// (Ex, Ex', Ey, Ey'), (Ez, Ez', Bx, Bx'), (By, By', Bz, Bz'). A cell's two z
+// nodes then arrive in three loads, as the register pairs that packed
+// products take. 48 bytes per node (28 MB on the GEM grid, L2-resident).
 struct PackedFields {
-  const float4 *eb4;
-  const float2 *eb2;
+  const float4 *eb;
 };
 
 // Device error word bits.

@@ -339,7 +339,7 @@ int run_copy_pipelined(Op op, Species *sp, struct particles *part, struct EMfiel
   SPB_CUDA(cudaEventRecord(sp->ev_in, sp->stream));
   for (int j = 0; j < NPIPE; ++j) SPB_CUDA(cudaStreamWaitEvent(sp->pipe[j], sp->ev_in, 0));
   const PushDev p = moves ? make_push(push_of(part, param)) : PushDev{};
-  const PackedFields F{ctx->d_eb4, ctx->d_eb2};
+  const PackedFields F{ctx->d_eb};
   long k = 0;
   for (long off = 0; off < n; off += PIPE_CHUNK, ++k) {
     cudaStream_t s = sp->pipe[k % NPIPE];
@@ -444,7 +444,7 @@ int run(Op op, struct particles *part, struct EMfield *field, struct interpDensS
       if (!f[a]) return fail(SPB_ERR_INVALID, "field array is null");
     if ((rc = spb_grid_set_fields(ctx, f, 0, sp->stream))) return rc;
     const PushDev p = make_push(push_of(part, param));
-    const PackedFields F{ctx->d_eb4, ctx->d_eb2};
+    const PackedFields F{ctx->d_eb};
     if (op == Op::Fused)
       rc = launch_plain_mover_interp(ctx->geom, p, F, sp->d[0], sp->d[1], sp->d[2], sp->d[3],
                                      sp->d[4], sp->d[5], sp->d[6], n, dm, sp->d_err, sp->stream);

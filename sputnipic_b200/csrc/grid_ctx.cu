@@ -125,14 +125,14 @@ int create_from_coords(const std::vector<float> &xn, const std::vector<float> &y
   c->nyn = (int)yn.size();
   c->nzn = (int)zn.size();
   c->nodes = (long)c->nxn * c->nyn * c->nzn;
-  const size_t ncoord = xn.size() + yn.size() + zn.size();
+  // the node coordinates, then (from an 8-byte boundary) their pairs
+  const size_t ncoord = xn.size() + yn.size() + zn.size(), pair0 = (ncoord + 1) & ~size_t(1);
   auto cleanup = [&](int rc) {
     spb_grid_destroy(c);
     return rc;
   };
-  if (cudaMalloc(&c->d_nodes, ncoord * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&c->d_eb4, c->nodes * sizeof(float4)) != cudaSuccess ||
-      cudaMalloc(&c->d_eb2, c->nodes * sizeof(float2)) != cudaSuccess ||
+  if (cudaMalloc(&c->d_nodes, (pair0 + 2 * ncoord) * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&c->d_eb, c->nodes * 3 * sizeof(float4)) != cudaSuccess ||
       cudaMalloc(&c->d_err, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     return cleanup(fail(SPB_ERR_ALLOC, "spb_grid_create: device allocation failed"));
@@ -140,7 +140,12 @@ int create_from_coords(const std::vector<float> &xn, const std::vector<float> &y
   std::vector<float> all(xn);
   all.insert(all.end(), yn.begin(), yn.end());
   all.insert(all.end(), zn.begin(), zn.end());
-  if (cudaMemcpy(c->d_nodes, all.data(), ncoord * sizeof(float), cudaMemcpyHostToDevice) !=
+  all.resize(pair0 + 2 * ncoord, 0.0f);
+  for (size_t i = 0; i < ncoord; ++i) {
+    all[pair0 + 2 * i] = i ? all[i - 1] : 0.0f;   // an axis's first pair is not read
+    all[pair0 + 2 * i + 1] = all[i];
+  }
+  if (cudaMemcpy(c->d_nodes, all.data(), all.size() * sizeof(float), cudaMemcpyHostToDevice) !=
           cudaSuccess ||
       cudaMemset(c->d_err, 0, sizeof(int)) != cudaSuccess ||
       cudaStreamSynchronize(nullptr) != cudaSuccess)   // the caller's stream may not wait for it
@@ -162,6 +167,22 @@ int create_from_coords(const std::vector<float> &xn, const std::vector<float> &y
   g.xn = c->d_nodes;
   g.yn = c->d_nodes + xn.size();
   g.zn = c->d_nodes + xn.size() + yn.size();
+  g.xp = reinterpret_cast<const float2 *>(c->d_nodes + pair0);
+  g.yp = g.xp + xn.size();
+  g.zp = g.yp + yn.size();
+  auto below = [](double L) {
+    float f = (float)L;
+    return (double)f > L ? std::nextafter(f, -INFINITY) : f;
+  };
+  g.Lfx = below(Lx);
+  g.Lfy = below(Ly);
+  g.Lfz = below(Lz);
+  g.nxf = (float)(g.nxn - 2);
+  g.nyf = (float)(g.nyn - 2);
+  g.nzf = (float)(g.nzn - 2);
+  const int most = 1 << 22;
+  g.float_cells = xStart == 0.0 && yStart == 0.0 && zStart == 0.0 && g.nxn < most &&
+                  g.nyn < most && g.nzn < most;
   *out = c;
   return SPB_OK;
 }
@@ -213,8 +234,7 @@ extern "C" int spb_grid_create_uniform(int nxc, int nyc, int nzc, double Lx, dou
 extern "C" void spb_grid_destroy(spb_grid_ctx *c) {
   if (!c) return;
   cudaFree(c->d_nodes);
-  cudaFree(c->d_eb4);
-  cudaFree(c->d_eb2);
+  cudaFree(c->d_eb);
   cudaFree(c->d_stage);
   cudaFree(c->d_net);
   cudaFree(c->d_err);
@@ -245,7 +265,7 @@ extern "C" int spb_grid_set_fields(spb_grid_ctx *c, const float *const fields[6]
       src[f] = c->d_stage + f * c->nodes;
     }
   }
-  int rc = launch_pack_fields(src, c->d_eb4, c->d_eb2, c->nodes, s);
+  int rc = launch_pack_fields(src, c->d_eb, c->nodes, c->nzn, s);
   if (rc) return rc;
   c->launches++;
   c->fields_set = true;
@@ -270,7 +290,7 @@ extern "C" int spb_grid_mover(spb_grid_ctx *c, const spb_push *push, float *x, f
   if (n < 0 || (n > 0 && (!x || !y || !z || !u || !v || !w)))
     return fail(SPB_ERR_INVALID, "spb_grid_mover: bad particle arrays");
   const PushDev p = make_push(*push);
-  int rc = launch_plain_mover(c->geom, p, PackedFields{c->d_eb4, c->d_eb2}, x, y, z, u, v, w, n,
+  int rc = launch_plain_mover(c->geom, p, PackedFields{c->d_eb}, x, y, z, u, v, w, n,
                               c->d_err, (cudaStream_t)stream);
   if (!rc && n > 0) c->launches++;
   return rc;
@@ -302,7 +322,7 @@ extern "C" int spb_grid_mover_interp(spb_grid_ctx *c, const spb_push *push, floa
     return fail(SPB_ERR_INVALID, "spb_grid_mover_interp: bad particle arrays");
   const PushDev p = make_push(*push);
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = launch_plain_mover_interp(c->geom, p, PackedFields{c->d_eb4, c->d_eb2}, x, y, z, u, v,
+  int rc = launch_plain_mover_interp(c->geom, p, PackedFields{c->d_eb}, x, y, z, u, v,
                                      w, q, n, mom, c->d_err, st);
   if (!rc && n > 0) c->launches += 2;
   return rc;

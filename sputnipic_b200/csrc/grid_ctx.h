@@ -11,9 +11,8 @@ struct spb_grid_ctx {
   int nxn = 0, nyn = 0, nzn = 0;
   long nodes = 0;
   spb::GeomDev geom{};
-  float *d_nodes = nullptr;      // xn | yn | zn
-  float4 *d_eb4 = nullptr;       // packed fields (Ex, Ey, Ez, Bx)
-  float2 *d_eb2 = nullptr;       // packed fields (By, Bz)
+  float *d_nodes = nullptr;      // xn | yn | zn, then their pairs
+  float4 *d_eb = nullptr;        // packed fields (PackedFields)
   float *d_stage = nullptr;      // 6*nodes staging for host field uploads
   float *d_net = nullptr;        // 10*nodes: net densities (sum over species)
   int *d_err = nullptr;

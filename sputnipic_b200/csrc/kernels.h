@@ -6,7 +6,7 @@
 namespace spb {
 
 // plain_kernels.cu
-int launch_pack_fields(const float *const f[6], float4 *eb4, float2 *eb2, long nodes,
+int launch_pack_fields(const float *const f[6], float4 *eb, long nodes, int nzn,
                        cudaStream_t s);
 int launch_plain_mover(const GeomDev &g, const PushDev &p, const PackedFields &F, float *x,
                        float *y, float *z, float *u, float *v, float *w, long n, int *err,

@@ -21,6 +21,7 @@
 #include "warp_sum.cuh"
 
 #include <atomic>
+#include <type_traits>
 
 namespace spb {
 
@@ -113,51 +114,133 @@ __device__ __forceinline__ void bc_axis_v(float &pos, float &vel, double L, int 
   }
 }
 
+// The mover's three cell indices, clamped to the node array. FLOAT_CELLS
+// (GeomDev::float_cells): the reference's double product of two floats is
+// exact, so a float product rounded toward zero has the same integer part
+// (every integer below 2^24 is a float, and rounding cannot cross one), and
+// the same comparisons with the integers -2 and n - 2 hold: cells outside the
+// node array (and NaN) take the general path, which flags them.
+template <bool FLOAT_CELLS>
+__device__ __forceinline__ void cell_index(const GeomDev &g, float x, float y, float z, int &ix,
+                                           int &iy, int &iz, int &bad) {
+  if (FLOAT_CELLS) {
+    const float px = __fmul_rz(x, g.invdx), py = __fmul_rz(y, g.invdy),
+                pz = __fmul_rz(z, g.invdz);
+    if (px > -2.0f && px < g.nxf && py > -2.0f && py < g.nyf && pz > -2.0f && pz < g.nzf) {
+      ix = 2 + __float2int_rz(px);
+      iy = 2 + __float2int_rz(py);
+      iz = 2 + __float2int_rz(pz);
+      return;
+    }
+  }
+  ix = clamp_cell(cell_trunc(x, g.xStart, g.invdx, g.nxn), g.nxn, bad);
+  iy = clamp_cell(cell_trunc(y, g.yStart, g.invdy, g.nyn), g.nyn, bad);
+  iz = clamp_cell(cell_trunc(z, g.zStart, g.invdz, g.nzn), g.nzn, bad);
+}
+
+// (float)(1.0 / (1.0 + (double)o)), bit for bit, o >= 0. An approximate float
+// reciprocal r of d = 1 + o and one third-order Newton step in double,
+// r (1 + e + e^2) with e = 1 - d r, give the quotient to within one unit in
+// its last place (e < 2^-21, so e^3 is far below it). Rounded to float that is
+// the rounded quotient unless the quotient lies within two units of the
+// midpoint of two floats; those, and o so large that r loses its precision
+// (or NaN), take the division itself.
+__device__ __forceinline__ float inv_one_plus(float o) {
+  const double d = 1.0 + (double)o;
+  float r0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(1.0f + o));
+  const double r = (double)r0;
+  const double e = __fma_rn(-d, r, 1.0);
+  double q = __fma_rn(r, __fma_rn(e, e, e), r);
+  // the bits of a double below a float's last one
+  const unsigned low = (unsigned)__double2loint(q) & 0x1fffffffu;
+  if (!(o < 1e18f) || low - 0x0ffffffeu <= 4u) q = 1.0 / d;
+  return (float)q;
+}
+
 // One particle of mover_PC (src/Mover.cpp:33-157); BCV = 1 gives mover_PC_V's
 // boundary handling instead.
-template <int BCV>
+//
+// Every result is the reference's, bit for bit; what its mixed arithmetic
+// computes in double is formed in float where that is provably the same:
+//   - the cell index: cell_index; 1 / (1 + omdtsq): inv_one_plus;
+//   - 2 upt - u in double, then to float: the difference of two floats is
+//     exact in double unless their exponents lie 30 or more apart, and then
+//     both roundings give the larger one, so one fused multiply-add (which
+//     rounds the exact difference once) is the same;
+//   - x > L: a float is above L exactly if it is above the largest float not
+//     above L.
+// The six field sums add c = 0 (the upper z node) before c = 1, as the
+// reference's loop does, and each product is rounded before it is added: the
+// products come from packed multiplies over the two z nodes, the sums from
+// scalar adds.
+//
+// The cell's eight nodes stay in registers over the iterations: most predicted
+// positions stay in the particle's cell, and only the lanes that left it load
+// again. The L1's data stage delivers 48 passes per warp and gather when the
+// lanes share a cell and two to three times that when the arrays have drifted
+// from cell order (it was 95 % busy then), so what the later iterations do not
+// load counts twice.
+template <int BCV, bool FLOAT_CELLS, int NITER>
 __device__ __forceinline__ void move_one(const GeomDev &g, const PushDev &p,
                                          const PackedFields &F, float &x, float &y,
                                          float &z, float &u, float &v, float &w,
                                          int &bad) {
   const float xpt = x, ypt = y, zpt = z;
-  const float qomdt2 = p.qomdt2;
+  const float qomdt2 = p.qomdt2, q2 = qomdt2 * qomdt2;
   float upt = 0.0f, vpt = 0.0f, wpt = 0.0f;
   float xc = x, yc = y, zc = z;
   const int sx = g.nyn * g.nzn, sy = g.nzn;   // nodes < 2^31 (spb_grid_create)
-  for (int it = 0; it < p.niter; ++it) {
-    const int ix = clamp_cell(cell_trunc(xc, g.xStart, g.invdx, g.nxn), g.nxn, bad);
-    const int iy = clamp_cell(cell_trunc(yc, g.yStart, g.invdy, g.nyn), g.nyn, bad);
-    const int iz = clamp_cell(cell_trunc(zc, g.zStart, g.invdz, g.nzn), g.nzn, bad);
-    const float xi[2] = {xc - __ldg(g.xn + ix - 1), __ldg(g.xn + ix) - xc};
-    const float eta[2] = {yc - __ldg(g.yn + iy - 1), __ldg(g.yn + iy) - yc};
-    const float zeta[2] = {zc - __ldg(g.zn + iz - 1), __ldg(g.zn + iz) - zc};
+  const float2 inv2 = make_float2(g.invVOL, g.invVOL);
+  int held = -1;        // cell whose eight nodes f holds
+  float4 f[12];
+#pragma unroll
+  for (int i = 0; i < 12; ++i) f[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int niter = NITER ? NITER : p.niter;
+#pragma unroll(NITER ? NITER : 1)
+  for (int it = 0; it < niter; ++it) {
+    int ix, iy, iz;
+    cell_index<FLOAT_CELLS>(g, xc, yc, zc, ix, iy, iz, bad);
+    const float2 xp = __ldg(g.xp + ix), yp = __ldg(g.yp + iy), zp = __ldg(g.zp + iz);
+    const float xi[2] = {xc - xp.x, xp.y - xc};
+    const float2 eta = make_float2(yc - yp.x, yp.y - yc);
+    const float2 zeta = make_float2(zc - zp.x, zp.y - zc);
     float Ex = 0.0f, Ey = 0.0f, Ez = 0.0f, Bx = 0.0f, By = 0.0f, Bz = 0.0f;
     const int base = ix * sx + iy * sy + iz;
+    if (base != held) {
+      held = base;
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+      for (int r = 0; r < 4; ++r) {
+        const float4 *row = F.eb + 3 * (long)(base - (r >> 1) * sx - (r & 1) * sy);
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
+        for (int k = 0; k < 3; ++k) f[3 * r + k] = __ldg(row + k);
+      }
+    }
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const float wgt = xi[a] * eta[b] * zeta[c] * g.invVOL;
-          const int n = base - a * sx - b * sy - c;
-          const float4 f4 = __ldg(F.eb4 + n);
-          const float2 f2 = __ldg(F.eb2 + n);
-          // the six products as three packed multiplies, summed one by one
-          const float2 w2 = make_float2(wgt, wgt);
-          const float2 pxy = mul2_rn(w2, make_float2(f4.x, f4.y));
-          const float2 pzx = mul2_rn(w2, make_float2(f4.z, f4.w));
-          const float2 pyz = mul2_rn(w2, f2);
-          Ex += pxy.x;
-          Ey += pxy.y;
-          Ez += pzx.x;
-          Bx += pzx.y;
-          By += pyz.x;
-          Bz += pyz.y;
-        }
-    const float omdtsq = qomdt2 * qomdt2 * (Bx * Bx + By * By + Bz * Bz);
-    const float denom = (float)(1.0 / (1.0 + (double)omdtsq));
+    for (int a = 0; a < 2; ++a) {
+      const float2 xe = mul2_rn(make_float2(xi[a], xi[a]), eta);
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const float s = b ? xe.y : xe.x;
+        // the weights of the two z nodes
+        const float2 w2 = mul2_rn(mul2_rn(make_float2(s, s), zeta), inv2);
+        const float4 f0 = f[6 * a + 3 * b], f1 = f[6 * a + 3 * b + 1], f2 = f[6 * a + 3 * b + 2];
+        const float2 ex = mul2_rn(w2, make_float2(f0.x, f0.y));
+        const float2 ey = mul2_rn(w2, make_float2(f0.z, f0.w));
+        const float2 ez = mul2_rn(w2, make_float2(f1.x, f1.y));
+        const float2 bx = mul2_rn(w2, make_float2(f1.z, f1.w));
+        const float2 by = mul2_rn(w2, make_float2(f2.x, f2.y));
+        const float2 bz = mul2_rn(w2, make_float2(f2.z, f2.w));
+        Ex = Ex + ex.x + ex.y;
+        Ey = Ey + ey.x + ey.y;
+        Ez = Ez + ez.x + ez.y;
+        Bx = Bx + bx.x + bx.y;
+        By = By + by.x + by.y;
+        Bz = Bz + bz.x + bz.y;
+      }
+    }
+    const float omdtsq = q2 * (Bx * Bx + By * By + Bz * Bz);
+    const float denom = inv_one_plus(omdtsq);
     const float ut = u + qomdt2 * Ex;
     const float vt = v + qomdt2 * Ey;
     const float wt = w + qomdt2 * Ez;
@@ -169,21 +252,24 @@ __device__ __forceinline__ void move_one(const GeomDev &g, const PushDev &p,
     yc = ypt + vpt * p.dto2;
     zc = zpt + wpt * p.dto2;
   }
-  u = (float)(2.0 * (double)upt - (double)u);
-  v = (float)(2.0 * (double)vpt - (double)v);
-  w = (float)(2.0 * (double)wpt - (double)w);
+  u = __fmaf_rn(2.0f, upt, -u);
+  v = __fmaf_rn(2.0f, vpt, -v);
+  w = __fmaf_rn(2.0f, wpt, -w);
   x = xpt + upt * p.dt_sub;
   y = ypt + vpt * p.dt_sub;
   z = zpt + wpt * p.dt_sub;
-  if (BCV == 0) {
-    bc_axis(x, u, g.Lx, p.periodic[0]);
-    bc_axis(y, v, g.Ly, p.periodic[1]);
-    bc_axis(z, w, g.Lz, p.periodic[2]);
-  } else {
-    bc_axis_v(x, u, g.Lx, p.periodic[0]);
-    bc_axis_v(y, v, g.Ly, p.periodic[1]);
-    bc_axis_v(z, w, g.Lz, p.periodic[2]);
-  }
+  // a particle inside [0, L] is left alone by both boundary conditions
+  auto bc = [&](float &pos, float &vel, float Lf, double L, int periodic) {
+    if (pos > Lf || pos < 0.0f) {
+      if (BCV == 0)
+        bc_axis(pos, vel, L, periodic);
+      else
+        bc_axis_v(pos, vel, L, periodic);
+    }
+  };
+  bc(x, u, g.Lfx, g.Lx, p.periodic[0]);
+  bc(y, v, g.Lfy, g.Ly, p.periodic[1]);
+  bc(z, w, g.Lfz, g.Lz, p.periodic[2]);
 }
 
 // The 40 summands of one x half of a particle (src/Mover.cpp:399-570), each
@@ -835,26 +921,36 @@ __global__ void __launch_bounds__(TPB) k_pack_fields(const float *__restrict__ e
                                                      const float *__restrict__ bx,
                                                      const float *__restrict__ by,
                                                      const float *__restrict__ bz,
-                                                     float4 *__restrict__ eb4,
-                                                     float2 *__restrict__ eb2, long nodes) {
+                                                     float4 *__restrict__ eb, long nodes,
+                                                     int nzn) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nodes;
        i += (long)gridDim.x * blockDim.x) {
-    eb4[i] = make_float4(ex[i], ey[i], ez[i], bx[i]);
-    eb2[i] = make_float2(by[i], bz[i]);
+    const long l = i % nzn ? i - 1 : i;   // the node below (a row's first is never read)
+    eb[3 * i] = make_float4(ex[i], ex[l], ey[i], ey[l]);
+    eb[3 * i + 1] = make_float4(ez[i], ez[l], bx[i], bx[l]);
+    eb[3 * i + 2] = make_float4(by[i], by[l], bz[i], bz[l]);
   }
 }
 
-template <int BCV>
-__global__ void __launch_bounds__(TPB) k_plain_mover(GeomDev g, PushDev p, PackedFields F,
+// Seven CTAs of 128 threads per SM (72 registers, 44 bytes of spills): the
+// pass is bound by the L1's data stage and by issue alike, and 28 warps keep
+// both busier than 24 without spills (3 to 4 % slower near cell order, as much
+// faster in long drifted arrays) or 32 with fewer nodes held. 65.5M electrons of
+// the GEM workload up to 15 steps after their arrays were in cell order: 2663 ->
+// 2300 us with the packing of the fields; 2.4M
+// electrons some cycles after the last sort: 166 -> 133 us.
+constexpr int MOVER_TPB = 128;
+template <int BCV, bool FLOAT_CELLS, int NITER>
+__global__ void __launch_bounds__(MOVER_TPB, 7) k_plain_mover(GeomDev g, PushDev p, PackedFields F,
                                                      float *__restrict__ x, float *__restrict__ y,
                                                      float *__restrict__ z, float *__restrict__ u,
                                                      float *__restrict__ v, float *__restrict__ w,
                                                      long n, int *__restrict__ err) {
-  const long i = blockIdx.x * (long)TPB + threadIdx.x;
+  const long i = blockIdx.x * (long)MOVER_TPB + threadIdx.x;
   if (i >= n) return;
   float px = x[i], py = y[i], pz = z[i], pu = u[i], pv = v[i], pw = w[i];
   int bad = 0;
-  move_one<BCV>(g, p, F, px, py, pz, pu, pv, pw, bad);
+  move_one<BCV, FLOAT_CELLS, NITER>(g, p, F, px, py, pz, pu, pv, pw, bad);
   x[i] = px;
   y[i] = py;
   z[i] = pz;
@@ -895,7 +991,7 @@ __global__ void __launch_bounds__(TPB) k_plain_mover_interp(
   int bad = 0;
   if (valid) {
     float px = x[i], py = y[i], pz = z[i], pu = u[i], pv = v[i], pw = w[i];
-    move_one<0>(g, p, F, px, py, pz, pu, pv, pw, bad);
+    move_one<0, false, 0>(g, p, F, px, py, pz, pu, pv, pw, bad);
     x[i] = px;
     y[i] = py;
     z[i] = pz;
@@ -955,10 +1051,10 @@ constexpr long P2S_MIN = 65536;
 
 }  // namespace
 
-int launch_pack_fields(const float *const f[6], float4 *eb4, float2 *eb2, long nodes,
+int launch_pack_fields(const float *const f[6], float4 *eb, long nodes, int nzn,
                        cudaStream_t s) {
   const unsigned blocks = (unsigned)std::min<long>(ceil_div(nodes, TPB), 4096);
-  k_pack_fields<<<blocks, TPB, 0, s>>>(f[0], f[1], f[2], f[3], f[4], f[5], eb4, eb2, nodes);
+  k_pack_fields<<<blocks, TPB, 0, s>>>(f[0], f[1], f[2], f[3], f[4], f[5], eb, nodes, nzn);
   SPB_CUDA(cudaGetLastError());
   g_launches++;
   return SPB_OK;
@@ -968,10 +1064,16 @@ int launch_plain_mover(const GeomDev &g, const PushDev &p, const PackedFields &F
                        float *y, float *z, float *u, float *v, float *w, long n, int *err,
                        cudaStream_t s, int bc_variant) {
   if (n <= 0) return SPB_OK;
-  if (bc_variant == 0)
-    k_plain_mover<0><<<blocks_for(n), TPB, 0, s>>>(g, p, F, x, y, z, u, v, w, n, err);
-  else
-    k_plain_mover<1><<<blocks_for(n), TPB, 0, s>>>(g, p, F, x, y, z, u, v, w, n, err);
+  // three iterations, the usual number, unrolled
+  auto pick = [&](auto bcv) {
+    constexpr int B = decltype(bcv)::value;
+    if (!g.float_cells) return k_plain_mover<B, false, 0>;
+    return p.niter == 3 ? k_plain_mover<B, true, 3> : k_plain_mover<B, true, 0>;
+  };
+  auto *const kernel = bc_variant == 0 ? pick(std::integral_constant<int, 0>())
+                                       : pick(std::integral_constant<int, 1>());
+  kernel<<<(unsigned)ceil_div(n, MOVER_TPB), MOVER_TPB, 0, s>>>(g, p, F, x, y, z, u, v, w, n,
+                                                              err);
   SPB_CUDA(cudaGetLastError());
   g_launches++;
   return SPB_OK;
