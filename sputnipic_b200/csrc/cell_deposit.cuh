@@ -91,13 +91,14 @@ struct PairOf<double> {
   using type = double2;
 };
 __device__ __forceinline__ float2 add_pair(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ double2 add_pair(double2 a, double2 b) {
-  return make_double2(a.x + b.x, a.y + b.y);
+template <typename T2>
+__device__ __forceinline__ double2 add_pair(double2 a, T2 b) {
+  return make_double2(a.x + (double)b.x, a.y + (double)b.y);
 }
 
 // Each node's sum of the totals of its (up to 8) cells in the tile, handed to
-// emit(bx, by, bz, sum[5]) (sum[k]: moments k and k + 5; the node's position
-// counted from the tile's lower corner). All threads of the CTA call, after a
+// emit(bx, by, bz, sum[5]) (sum[k]: moments k and k + 5, summed in A; the node's
+// position counted from the tile's lower corner). All threads of the CTA call, after a
 // barrier behind the totals' stores. A thread takes a node and its ten
 // moments: the node's position and which of its cells lie in the tile are
 // formed once, the cells' pairs lie at fixed offsets from one address, and one
@@ -105,9 +106,10 @@ __device__ __forceinline__ double2 add_pair(double2 a, double2 b) {
 // spent most of its instructions on those addresses; the precision form's
 // deposit of the GEM grid, 4 species: 396 -> 323 us at 8 particles per cell,
 // 697 -> 636 us at 27, 2100 -> 2050 us at 125.)
-template <int TX, int TY, int TZ, int NT, typename T, typename Emit>
+template <int TX, int TY, int TZ, int NT, typename T, typename A, typename Emit>
 __device__ __forceinline__ void node_sums(const typename PairOf<T>::type *sCell, Emit emit) {
   using T2 = typename PairOf<T>::type;
+  using A2 = typename PairOf<A>::type;
   constexpr int NX = TX + 1, NY = TY + 1, NZ = TZ + 1, NB = NX * NY * NZ;
   constexpr int TC = TX * TY * TZ;
   for (int nb = threadIdx.x; nb < NB; nb += NT) {
@@ -115,9 +117,9 @@ __device__ __forceinline__ void node_sums(const typename PairOf<T>::type *sCell,
     // the cell above the node on an axis (corner bit 0) or the one below it (1)
     const bool inx[2] = {bx < TX, bx > 0}, iny[2] = {by < TY, by > 0}, inz[2] = {bz < TZ, bz > 0};
     const T2 *at = sCell + (bx * TY + by) * TZ + bz;
-    T2 sum[5];
+    A2 sum[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) sum[k].x = sum[k].y = (T)0;
+    for (int k = 0; k < 5; ++k) sum[k].x = sum[k].y = (A)0;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int a = e >> 2, b = (e >> 1) & 1, c = e & 1;

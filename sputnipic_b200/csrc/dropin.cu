@@ -331,10 +331,12 @@ int run_copy_pipelined(Op op, Species *sp, struct particles *part, struct EMfiel
       if (!f[a]) return fail(SPB_ERR_INVALID, "field array is null");
     if (int rc = spb_grid_set_fields(ctx, f, 0, sp->stream)) return rc;
   }
-  float *acc = nullptr;   // one accumulator for all chunks, folded once
+  float *acc = nullptr;   // the last chunk's accumulator
   if (deposits) {
     if (int rc = upload_moments(sp, ids, nodes, dev_mom, hm, dm)) return rc;
-    acc = plain_acc_alloc(ctx->geom, sp->stream);
+    // only a last chunk too small for the sorted deposit adds into one
+    if (n % PIPE_CHUNK && plain_wants_acc(n % PIPE_CHUNK))
+      acc = plain_acc_alloc(ctx->geom, sp->stream);
   }
   SPB_CUDA(cudaEventRecord(sp->ev_in, sp->stream));
   for (int j = 0; j < NPIPE; ++j) SPB_CUDA(cudaStreamWaitEvent(sp->pipe[j], sp->ev_in, 0));

@@ -36,9 +36,19 @@ void pool_free(void *p, cudaStream_t s);
 // stream-ordered pool on stream s, or nullptr when it cannot be had (the
 // deposits then add straight into the moment arrays).
 float *plain_acc_alloc(const GeomDev &g, cudaStream_t s);
+// Whether a deposit of n particles adds into an accumulator (the others go
+// through sorted_p2g straight into the moment arrays).
+bool plain_wants_acc(long n);
 // Adds the accumulator into mom[0..9] and returns it to the pool (nothing
 // for nullptr).
 int plain_acc_fold(float *acc, const GeomDev &g, float *const mom[10], cudaStream_t s);
+// plain_sorted_p2g.cu: the deposit in cell order. Deposits particles
+// 0 .. *done - 1 into mom; fewer than n only where scratch could not be had
+// for more (the caller deposits the rest another way).
+constexpr long SORTED_P2G_MIN = 65536;
+int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z, const float *u,
+               const float *v, const float *w, const float *q, long n, float *const mom[10],
+               int *err, cudaStream_t s, long *done);
 // interpP2G / mover_interp deposits into acc (mom when acc is nullptr).
 int launch_plain_p2g_into(const GeomDev &g, const float *x, const float *y, const float *z,
                           const float *u, const float *v, const float *w, const float *q, long n,

@@ -18,6 +18,8 @@
 // 128x64x64 cells).
 #include "bc_fold.cuh"
 #include "grid_ctx.h"
+#include "kernels.h"
+#include "plain_cells.cuh"
 #include "warp_sum.cuh"
 
 #include <atomic>
@@ -33,33 +35,6 @@ constexpr int TPB = 256;
 struct Moments10 {
   float *m[10];
 };
-
-// The double product (x - start) * inv, limited to [-8, n + 8] so that the
-// int conversion below never overflows (NaN maps to -8). Exact for every
-// position inside the grid, where the limit does not bite.
-__device__ __forceinline__ double cell_coord(float p, double start, float inv, int n) {
-  const double d = ((double)p - start) * (double)inv;
-  return fmin(fmax(d, -8.0), (double)n + 8.0);
-}
-
-// Reference cell index of the mover: 2 + int((x - xStart) * invdx), the
-// product in double, truncated toward zero (src/Mover.cpp:39-41).
-__device__ __forceinline__ int cell_trunc(float p, double start, float inv, int n) {
-  return 2 + __double2int_rz(cell_coord(p, start, inv, n));
-}
-
-// Reference cell index of the deposit: 2 + int(floor(...)) (src/Mover.cpp:399-401).
-__device__ __forceinline__ int cell_floor(float p, double start, float inv, int n) {
-  return 2 + __double2int_rd(cell_coord(p, start, inv, n));
-}
-
-// Keeps the node pair (i-1, i) inside [0, n-1]. The reference reads out of
-// bounds for such particles; here they are flagged and clamped.
-__device__ __forceinline__ int clamp_cell(int i, int n, int &bad) {
-  if (i < 1) { bad = 1; return 1; }
-  if (i > n - 1) { bad = 1; return n - 1; }
-  return i;
-}
 
 // x * y on a pair of floats, each half rounded to nearest on its own, as a
 // scalar float multiply rounds it. The mover adds the two halves with scalar
@@ -516,8 +491,8 @@ __device__ __forceinline__ Particle smem_particle(const GroupSmem &S, int j) {
   return Particle{S.p[0][j], S.p[1][j], S.p[2][j], S.p[3][j], S.p[4][j], S.p[5][j], S.p[6][j]};
 }
 
-// (Particles in the arrays' own order; cell-ordered input goes through
-// k_plain_p2g_runs instead.)
+// (Particles in the arrays' own order: deposits below P2S_MIN particles and
+// those whose scratch cannot be had; the others go through sorted_p2g.)
 template <bool ACC>
 __global__ void __launch_bounds__(GP_TPB) k_plain_p2g_grouped(
     GeomDev g, const float *__restrict__ x, const float *__restrict__ y,
@@ -651,270 +626,6 @@ __global__ void __launch_bounds__(GP_TPB) k_plain_p2g_grouped(
   if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
 }
 
-// The plain deposit over particles in cell order (a permutation from the cell
-// sort below). A CTA takes a chunk of RUN_CHUNK consecutive positions of the
-// permutation; while loading them it computes each particle's deposit cell
-// and its six node distances (xi0 = x - xn[ix-1], xi1 = xn[ix] - x, and so
-// on, src/Mover.cpp:399-410) once, into shared memory with u, v, w, q. Each
-// warp then takes an equal slice of the chunk: in the slice the particles of
-// one cell form runs, and a run of four or more is deposited as one group
-// (run_terms for both x halves, one warp reduction, 80 adds), shorter runs
-// particle by particle. A run that a slice or chunk boundary cuts is
-// deposited in parts.
-constexpr int RUN_TPB = 256;
-constexpr int RUN_PER_THREAD = 4;
-constexpr int RUN_CHUNK = RUN_TPB * RUN_PER_THREAD;
-static_assert(RUN_CHUNK == GP_CHUNK, "one grid size for both deposit kernels");
-
-struct RunSmem {
-  float d[10][RUN_CHUNK];   // xi0, xi1, eta0, eta1, zeta0, zeta1, u, v, w, q
-  int key[RUN_CHUNK];       // node-space cell
-};
-
-// half_terms from the stored node distances of particle j: the same 40
-// summands, each product in the reference's order (pairs of independent
-// products issued as one packed FP32x2 multiply). With ADD, a term's last
-// multiply may be fused into the packed sum that follows it (one rounding
-// instead of two); the moments are a reordered FP32 sum either way.
-template <bool ADD>
-__device__ __forceinline__ void run_terms(const GeomDev &g, const RunSmem &S, int j,
-                                          float2 (&t)[20], int lane, int a) {
-  const bool pb = lane & 8, pc = lane & 4;
-  const float xi0 = S.d[0][j], xi1 = S.d[1][j], eta0 = S.d[2][j], eta1 = S.d[3][j];
-  const float zeta0 = S.d[4][j], zeta1 = S.d[5][j];
-  const float u = S.d[6][j], v = S.d[7][j], w = S.d[8][j], q = S.d[9][j];
-  const float xia = (a ^ ((lane >> 4) & 1)) ? xi1 : xi0;
-  const float eta[2] = {pb ? eta1 : eta0, pb ? eta0 : eta1};
-  const float2 zeta = pc ? make_float2(zeta1, zeta0) : make_float2(zeta0, zeta1);
-  const float2 uu_vv = __fmul2_rn(make_float2(u, v), make_float2(u, v));
-  const float2 uv_vw = __fmul2_rn(make_float2(u, v), make_float2(v, w));
-  const float2 uw_ww = __fmul2_rn(make_float2(u, w), make_float2(w, w));
-  // factor pairs (moment k, moment k + 5); rhon's (1 * wgt) * inv is the
-  // reference's wgt * inv exactly
-  const float2 f[5] = {make_float2(1.0f, uv_vw.x), make_float2(u, uw_ww.x),
-                       make_float2(v, uu_vv.y), make_float2(w, uv_vw.y),
-                       make_float2(uu_vv.x, uw_ww.y)};
-  const float2 inv = make_float2(g.invVOL, g.invVOL);
-  const float qx = q * xia;
-#pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    const float qxe = qx * eta[b];
-    // ((q * xi * eta) * zeta) * invVOL for both z nodes
-    const float2 wgt = __fmul2_rn(__fmul2_rn(make_float2(qxe, qxe), zeta), inv);
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const float wc = c ? wgt.y : wgt.x;
-      const float2 w2 = make_float2(wc, wc);
-      float2 *o = t + (b * 2 + c) * 5;
-#pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        const float2 n = __fmul2_rn(__fmul2_rn(f[k], w2), inv);
-        o[k] = ADD ? __fadd2_rn(o[k], n) : n;
-      }
-    }
-  }
-}
-
-// deposit_lone from the stored node distances of particle j (all 32 lanes
-// call with the same j and key).
-template <bool ACC>
-__device__ __forceinline__ void run_lone(const GeomDev &g, const DepTarget &T, const RunSmem &S,
-                                         int j, int key) {
-  const int lane = threadIdx.x & 31;
-  const int sx = g.nyn * g.nzn, sy = g.nzn;
-  if (lane >= 24) return;
-  const int node = lane / 3, grp = lane % 3;
-  const int a = node >> 2, b = (node >> 1) & 1, c = node & 1;
-  const float inv = g.invVOL, u = S.d[6][j], v = S.d[7][j], w = S.d[8][j];
-  const float wgt = S.d[9][j] * S.d[a][j] * S.d[2 + b][j] * S.d[4 + c][j] * inv;
-  const float f0 = grp == 0 ? 1.0f : (grp == 1 ? u * u : v * w);
-  const float f1 = grp == 0 ? u : (grp == 1 ? u * v : w * w);
-  const float f2 = grp == 0 ? v : (grp == 1 ? u * w : 0.0f);
-  const float f3 = grp == 0 ? w : (grp == 1 ? v * v : 0.0f);
-  dep_add4<ACC>(T, key - a * sx - b * sy - c, grp, (f0 * wgt) * inv, (f1 * wgt) * inv,
-                (f2 * wgt) * inv, (f3 * wgt) * inv);
-}
-
-template <bool ACC>
-__global__ void __launch_bounds__(RUN_TPB, 3) k_plain_p2g_runs(
-    GeomDev g, const float *__restrict__ x, const float *__restrict__ y,
-    const float *__restrict__ z, const float *__restrict__ u, const float *__restrict__ v,
-    const float *__restrict__ w, const float *__restrict__ q, long n,
-    const unsigned *__restrict__ perm, const __grid_constant__ DepTarget T,
-    int *__restrict__ err) {
-  __shared__ RunSmem S;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long base = (long)blockIdx.x * RUN_CHUNK;
-  const int cnt = (int)min((long)RUN_CHUNK, n - base);
-  int bad = 0;
-#pragma unroll
-  for (int r = 0; r < RUN_PER_THREAD; ++r) {
-    const int j = tid + r * RUN_TPB;
-    if (j < cnt) {
-      const long i = perm[base + j];
-      const float px = x[i], py = y[i], pz = z[i];
-      const int ix = clamp_cell(cell_floor(px, g.xStart, g.invdx, g.nxn), g.nxn, bad);
-      const int iy = clamp_cell(cell_floor(py, g.yStart, g.invdy, g.nyn), g.nyn, bad);
-      const int iz = clamp_cell(cell_floor(pz, g.zStart, g.invdz, g.nzn), g.nzn, bad);
-      S.key[j] = (ix * g.nyn + iy) * g.nzn + iz;
-      S.d[0][j] = px - __ldg(g.xn + ix - 1);
-      S.d[1][j] = __ldg(g.xn + ix) - px;
-      S.d[2][j] = py - __ldg(g.yn + iy - 1);
-      S.d[3][j] = __ldg(g.yn + iy) - py;
-      S.d[4][j] = pz - __ldg(g.zn + iz - 1);
-      S.d[5][j] = __ldg(g.zn + iz) - pz;
-      S.d[6][j] = u[i];
-      S.d[7][j] = v[i];
-      S.d[8][j] = w[i];
-      S.d[9][j] = q[i];
-    }
-  }
-  __syncthreads();
-  const int sx = g.nyn * g.nzn, sy = g.nzn;
-  const int na = (lane >> 4) & 1, nb = (lane >> 3) & 1, nc = (lane >> 2) & 1;
-  const int mbase = 5 * ((lane >> 1) & 1);
-  const int lo = (lane & 1) ? 3 : 0, hi = (lane & 1) ? 5 : 3;
-  constexpr int PW = RUN_CHUNK / (RUN_TPB / 32);   // positions per warp
-  const int jend = min((warp + 1) * PW, cnt);
-#pragma unroll 1
-  for (int j = warp * PW; j < jend;) {
-    // the run of key S.key[j]: up to the first position with another key
-    const int key = S.key[j];
-    int e = jend;
-#pragma unroll 1
-    for (int b = j + 1; b < jend; b += 32) {
-      const int t = b + lane;
-      const unsigned m = __ballot_sync(FULL, t < jend && S.key[t] != key);
-      if (m) {
-        e = b + __ffs(m) - 1;
-        break;
-      }
-    }
-    const int c = e - j;
-    if (c <= 3) {
-      for (int m = 0; m < c; ++m) run_lone<ACC>(g, T, S, j + m, key);
-    } else {
-      float2 t[20];
-#pragma unroll
-      for (int i = 0; i < 20; ++i) t[i] = make_float2(0.0f, 0.0f);
-      for (int m = lane; m < c; m += 32) run_terms<true>(g, S, j + m, t, lane, 1);
-#pragma unroll
-      for (int i = 0; i < 20; ++i) t[i] = shfl_xor2(t[i], 16);
-      for (int m = lane; m < c; m += 32) run_terms<true>(g, S, j + m, t, lane, 0);
-      float r[5];
-      warp_sum80_tail(t, r, lane);
-      const int node = key - na * sx - nb * sy - nc;
-#pragma unroll
-      for (int i = 0; i < 5; ++i)
-        if (i >= lo && i < hi) dep_add<ACC>(T, node, mbase + i, r[i]);
-    }
-    j = e;
-  }
-  if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
-}
-
-// The plain deposit's cell sort: a counting sort of (cell, index) pairs by
-// the deposit's own cell (the node-space floor cell of src/Mover.cpp:399-401).
-// Keys and per-cell counts (one atomic per distinct cell of a warp) ...
-__global__ void __launch_bounds__(TPB) k_p2g_keys(GeomDev g, const float *__restrict__ x,
-                                                  const float *__restrict__ y,
-                                                  const float *__restrict__ z, long n,
-                                                  unsigned *__restrict__ key,
-                                                  unsigned *__restrict__ count) {
-  const int lane = threadIdx.x & 31;
-  int ignored = 0;   // the deposit flags cells off the node array
-  for (long base = (long)blockIdx.x * TPB; base < n; base += (long)gridDim.x * TPB) {
-    const long i = base + threadIdx.x;
-    const bool valid = i < n;
-    unsigned k = 0xffffffffu;
-    if (valid) {
-      const int ix = clamp_cell(cell_floor(x[i], g.xStart, g.invdx, g.nxn), g.nxn, ignored);
-      const int iy = clamp_cell(cell_floor(y[i], g.yStart, g.invdy, g.nyn), g.nyn, ignored);
-      const int iz = clamp_cell(cell_floor(z[i], g.zStart, g.invdz, g.nzn), g.nzn, ignored);
-      k = (unsigned)((ix * g.nyn + iy) * g.nzn + iz);
-      key[i] = k;
-    }
-    const unsigned peers = __match_any_sync(FULL, k);
-    if (valid && lane == __ffs(peers) - 1) atomicAdd(count + k, (unsigned)__popc(peers));
-  }
-}
-
-// ... an exclusive scan of the counts into the cells' first positions (three
-// passes over blocks of P2S_B) ...
-constexpr int P2S_B = 1024;
-__device__ __forceinline__ unsigned p2s_block_scan(unsigned v, unsigned *ws, unsigned &total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned xs = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned t = __shfl_up_sync(FULL, xs, o);
-    if (lane >= o) xs += t;
-  }
-  if (lane == 31) ws[warp] = xs;
-  __syncthreads();
-  if (warp == 0) {
-    unsigned s = ws[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned t = __shfl_up_sync(FULL, s, o);
-      if (lane >= o) s += t;
-    }
-    ws[lane] = s;
-  }
-  __syncthreads();
-  const unsigned pre = warp ? ws[warp - 1] : 0u;
-  total = ws[31];
-  __syncthreads();
-  return pre + xs - v;
-}
-
-__global__ void __launch_bounds__(P2S_B) k_p2s_scan_blocks(const unsigned *in, long m,
-                                                           unsigned *out, unsigned *bsum) {
-  __shared__ unsigned ws[32];
-  const long i = blockIdx.x * (long)P2S_B + threadIdx.x;
-  unsigned total;
-  const unsigned ex = p2s_block_scan(i < m ? in[i] : 0u, ws, total);
-  if (i < m) out[i] = ex;
-  if (threadIdx.x == 0) bsum[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(P2S_B) k_p2s_scan_sums(unsigned *bsum, int nb) {
-  __shared__ unsigned ws[32];
-  unsigned carry = 0;
-  for (int b = 0; b < nb; b += P2S_B) {
-    const int i = b + threadIdx.x;
-    unsigned total;
-    const unsigned ex = p2s_block_scan(i < nb ? bsum[i] : 0u, ws, total);
-    if (i < nb) bsum[i] = ex + carry;
-    carry += total;
-  }
-}
-
-__global__ void __launch_bounds__(P2S_B) k_p2s_scan_add(unsigned *out, long m,
-                                                        const unsigned *bsum) {
-  const long i = blockIdx.x * (long)P2S_B + threadIdx.x;
-  if (i < m) out[i] += bsum[blockIdx.x];
-}
-
-// ... and every index at its cell's next free position (cursor: the first
-// positions, advanced; the order inside a cell is the atomics').
-__global__ void __launch_bounds__(TPB) k_p2g_scatter(const unsigned *__restrict__ key, long n,
-                                                     unsigned *__restrict__ cursor,
-                                                     unsigned *__restrict__ perm) {
-  const int lane = threadIdx.x & 31;
-  for (long base = (long)blockIdx.x * TPB; base < n; base += (long)gridDim.x * TPB) {
-    const long i = base + threadIdx.x;
-    const bool valid = i < n;
-    const unsigned k = valid ? key[i] : 0xffffffffu;
-    const unsigned peers = __match_any_sync(FULL, k);
-    const int leader = __ffs(peers) - 1;
-    unsigned first = 0;
-    if (valid && lane == leader) first = atomicAdd(cursor + k, (unsigned)__popc(peers));
-    first = __shfl_sync(FULL, first, leader);
-    if (valid) perm[first + __popc(peers & ((1u << lane) - 1u))] = (unsigned)i;
-  }
-}
-
 __global__ void __launch_bounds__(TPB) k_pack_fields(const float *__restrict__ ex,
                                                      const float *__restrict__ ey,
                                                      const float *__restrict__ ez,
@@ -957,50 +668,6 @@ __global__ void __launch_bounds__(MOVER_TPB, 7) k_plain_mover(GeomDev g, PushDev
   u[i] = pu;
   v[i] = pv;
   w[i] = pw;
-  if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
-}
-
-template <bool ACC>
-__global__ void __launch_bounds__(TPB) k_plain_p2g(GeomDev g, const float *__restrict__ x,
-                                                   const float *__restrict__ y,
-                                                   const float *__restrict__ z,
-                                                   const float *__restrict__ u,
-                                                   const float *__restrict__ v,
-                                                   const float *__restrict__ w,
-                                                   const float *__restrict__ q, long n,
-                                                   const __grid_constant__ DepTarget T,
-                                                   int *__restrict__ err) {
-  const long i = blockIdx.x * (long)TPB + threadIdx.x;
-  const bool valid = i < n;
-  Particle p{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (valid) p = Particle{x[i], y[i], z[i], u[i], v[i], w[i], q[i]};
-  int bad = 0;
-  deposit_warp<ACC>(g, T, valid, p, bad);
-  if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
-}
-
-template <bool ACC>
-__global__ void __launch_bounds__(TPB) k_plain_mover_interp(
-    GeomDev g, PushDev p, PackedFields F, float *__restrict__ x, float *__restrict__ y,
-    float *__restrict__ z, float *__restrict__ u, float *__restrict__ v,
-    float *__restrict__ w, const float *__restrict__ q, long n,
-    const __grid_constant__ DepTarget T, int *__restrict__ err) {
-  const long i = blockIdx.x * (long)TPB + threadIdx.x;
-  const bool valid = i < n;
-  Particle pt{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  int bad = 0;
-  if (valid) {
-    float px = x[i], py = y[i], pz = z[i], pu = u[i], pv = v[i], pw = w[i];
-    move_one<0, false, 0>(g, p, F, px, py, pz, pu, pv, pw, bad);
-    x[i] = px;
-    y[i] = py;
-    z[i] = pz;
-    u[i] = pu;
-    v[i] = pv;
-    w[i] = pw;
-    pt = Particle{px, py, pz, pu, pv, pw, q[i]};
-  }
-  deposit_warp<ACC>(g, T, valid, pt, bad);
   if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
 }
 
@@ -1047,7 +714,7 @@ __global__ void __launch_bounds__(TPB) k_bc_fold(const __grid_constant__ Moments
 inline unsigned blocks_for(long n) { return (unsigned)ceil_div(n, TPB); }
 
 // Deposits of at least this many particles sort them by cell first.
-constexpr long P2S_MIN = 65536;
+constexpr long P2S_MIN = SORTED_P2G_MIN;
 
 }  // namespace
 
@@ -1176,45 +843,15 @@ int launch_plain_p2g_into(const GeomDev &g, const float *x, const float *y, cons
                           const float *u, const float *v, const float *w, const float *q, long n,
                           float *acc, float *const mom[10], int *err, cudaStream_t s) {
   if (n <= 0) return SPB_OK;
+  long done = 0;   // particles deposited in cell order
+  if (n >= P2S_MIN)
+    if (int rc = sorted_p2g(g, x, y, z, u, v, w, q, n, mom, err, s, &done)) return rc;
+  if (done == n) return SPB_OK;
   const DepTarget T = target(acc, mom);
-  const unsigned chunks = (unsigned)ceil_div(n, GP_CHUNK);
-  // the particles in cell order first (above P2S_MIN; scratch from the
-  // device's pool, skipped if it cannot be had)
-  unsigned *scratch = nullptr, *perm = nullptr;
-  const long nodes = (long)g.nxn * g.nyn * g.nzn;
-  if (n >= P2S_MIN) {
-    const long nb = ceil_div(nodes, P2S_B);
-    keep_pool_memory();
-    const size_t words = (size_t)2 * n + 2 * nodes + nb;
-    if (cudaMallocAsync(reinterpret_cast<void **>(&scratch), words * sizeof(unsigned), s) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      scratch = nullptr;
-    }
-    if (scratch) {
-      unsigned *key = scratch, *pm = scratch + n, *count = pm + n, *first = count + nodes;
-      unsigned *bsum = first + nodes;
-      SPB_CUDA(cudaMemsetAsync(count, 0, nodes * sizeof(unsigned), s));
-      const unsigned blocks = (unsigned)std::min<long>(ceil_div(n, TPB), 148L * 16);
-      k_p2g_keys<<<blocks, TPB, 0, s>>>(g, x, y, z, n, key, count);
-      k_p2s_scan_blocks<<<(unsigned)nb, P2S_B, 0, s>>>(count, nodes, first, bsum);
-      k_p2s_scan_sums<<<1, P2S_B, 0, s>>>(bsum, (int)nb);
-      k_p2s_scan_add<<<(unsigned)nb, P2S_B, 0, s>>>(first, nodes, bsum);
-      k_p2g_scatter<<<blocks, TPB, 0, s>>>(key, n, first, pm);
-      SPB_CUDA(cudaGetLastError());
-      g_launches += 5;
-      perm = pm;
-    }
-  }
-  if (perm && acc)
-    k_plain_p2g_runs<true><<<chunks, RUN_TPB, 0, s>>>(g, x, y, z, u, v, w, q, n, perm, T, err);
-  else if (perm)
-    k_plain_p2g_runs<false><<<chunks, RUN_TPB, 0, s>>>(g, x, y, z, u, v, w, q, n, perm, T, err);
-  else if (acc)
-    k_plain_p2g_grouped<true><<<chunks, GP_TPB, 0, s>>>(g, x, y, z, u, v, w, q, n, T, err);
-  else
-    k_plain_p2g_grouped<false><<<chunks, GP_TPB, 0, s>>>(g, x, y, z, u, v, w, q, n, T, err);
-  if (scratch) cudaFreeAsync(scratch, s);
+  const unsigned chunks = (unsigned)ceil_div(n - done, GP_CHUNK);
+  auto *const kernel = acc ? k_plain_p2g_grouped<true> : k_plain_p2g_grouped<false>;
+  kernel<<<chunks, GP_TPB, 0, s>>>(g, x + done, y + done, z + done, u + done, v + done, w + done,
+                                   q + done, n - done, T, err);
   SPB_CUDA(cudaGetLastError());
   g_launches++;
   return SPB_OK;
@@ -1224,24 +861,17 @@ int launch_plain_mover_interp_into(const GeomDev &g, const PushDev &p, const Pac
                                    float *x, float *y, float *z, float *u, float *v, float *w,
                                    const float *q, long n, float *acc, float *const mom[10],
                                    int *err, cudaStream_t s) {
-  if (n <= 0) return SPB_OK;
-  const DepTarget T = target(acc, mom);
-  if (acc)
-    k_plain_mover_interp<true><<<blocks_for(n), TPB, 0, s>>>(g, p, F, x, y, z, u, v, w, q, n, T,
-                                                             err);
-  else
-    k_plain_mover_interp<false><<<blocks_for(n), TPB, 0, s>>>(g, p, F, x, y, z, u, v, w, q, n,
-                                                              T, err);
-  SPB_CUDA(cudaGetLastError());
-  g_launches++;
-  return SPB_OK;
+  if (int rc = launch_plain_mover(g, p, F, x, y, z, u, v, w, n, err, s)) return rc;
+  return launch_plain_p2g_into(g, x, y, z, u, v, w, q, n, acc, mom, err, s);
 }
+
+bool plain_wants_acc(long n) { return n < P2S_MIN; }
 
 int launch_plain_p2g(const GeomDev &g, const float *x, const float *y, const float *z,
                      const float *u, const float *v, const float *w, const float *q, long n,
                      float *const mom[10], int *err, cudaStream_t s) {
   if (n <= 0) return SPB_OK;
-  float *acc = plain_acc_alloc(g, s);
+  float *acc = plain_wants_acc(n) ? plain_acc_alloc(g, s) : nullptr;
   const int rc = launch_plain_p2g_into(g, x, y, z, u, v, w, q, n, acc, mom, err, s);
   if (rc) {
     if (acc) cudaFreeAsync(acc, s);
@@ -1254,14 +884,8 @@ int launch_plain_mover_interp(const GeomDev &g, const PushDev &p, const PackedFi
                               float *x, float *y, float *z, float *u, float *v, float *w,
                               const float *q, long n, float *const mom[10], int *err,
                               cudaStream_t s) {
-  if (n <= 0) return SPB_OK;
-  float *acc = plain_acc_alloc(g, s);
-  const int rc = launch_plain_mover_interp_into(g, p, F, x, y, z, u, v, w, q, n, acc, mom, err, s);
-  if (rc) {
-    if (acc) cudaFreeAsync(acc, s);
-    return rc;
-  }
-  return plain_acc_fold(acc, g, mom, s);
+  if (int rc = launch_plain_mover(g, p, F, x, y, z, u, v, w, n, err, s)) return rc;
+  return launch_plain_p2g(g, x, y, z, u, v, w, q, n, mom, err, s);
 }
 
 int launch_apply_bc_ids(int nxn, int nyn, int nzn, const int periodic[3],

@@ -967,7 +967,7 @@ __device__ __forceinline__ void add_node_sums(const CycleParams &P, double *__re
                                               const typename PairOf<T>::type *sCell, int c0x,
                                               int c0y, int c0z, double scale) {
   const long nodes = (long)P.nxn * P.nyn * P.nzn;
-  node_sums<TX, TY, TZ, NT, T>(
+  node_sums<TX, TY, TZ, NT, T, T>(
       sCell, [&](int bx, int by, int bz, const typename PairOf<T>::type(&sum)[5]) {
         double *to =
             mom + ((long)(c0x + bx + 1) * P.nyn + (c0y + by + 1)) * P.nzn + (c0z + bz + 1);

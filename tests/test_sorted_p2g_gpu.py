@@ -1,0 +1,118 @@
+"""The plain deposit in cell order (65,536 particles and more) against the oracle: sizes at the
+threshold and its remainders, grids smaller than a tile and longer than one, all particles in one
+cell, particles on nodes and walls, a domain that does not start at 0, positions off the grid, and
+more particles than one chunk holds. Bar: |gpu - ref| <= 32 eps32 sum |term| per node (the rounding
+bound of a reordered float sum, as in test_parity_plain_gpu.py)."""
+import numpy as np
+import pytest
+
+import oracle
+from sputnipic_b200 import workload as W
+
+pytestmark = pytest.mark.gpu
+EPS32 = float(np.finfo(np.float32).eps)
+
+
+def particles(rng, wl, n, where):
+    p = {}
+    for k, L, c in zip("xyz", (wl.Lx, wl.Ly, wl.Lz), (wl.nxc, wl.nyc, wl.nzc)):
+        if where == "one cell":
+            a = (c // 2 + rng.random(n)) * (L / c)
+        elif where == "nodes":
+            a = rng.integers(0, c + 1, n) * (L / c)
+        else:
+            a = rng.random(n) * L
+        a = a.astype(np.float32)
+        p[k] = np.where(a.astype(np.float64) > L, np.nextafter(a, np.float32(0)), a)
+    for k in "uvw":
+        p[k] = (0.05 * rng.standard_normal(n)).astype(np.float32)
+    p["q"] = rng.uniform(-1, 1, n).astype(np.float32)
+    return p
+
+
+def check(got, wl, p):
+    setup = oracle.setup_from(wl)
+    ref = [np.zeros(wl.nodes, np.float32) for _ in range(10)]
+    oracle.CpuOracle("restated", 32).interp_p2g(setup, p, ref)
+    a = {k: (np.abs(p[k]) if k in "uvwq" else p[k]).astype(np.float64) for k in "xyzuvwq"}
+    absm = [np.zeros(wl.nodes) for _ in range(10)]
+    oracle.CpuOracle("restated", 64).interp_p2g(setup, a, absm)
+    bad = np.abs(got.astype(np.float64) - np.stack(ref)) > 32 * EPS32 * np.stack(absm) + 1e-30
+    assert not bad.any(), f"{bad.sum()} moment entries outside the bound"
+
+
+def on_gpu(torch, p):
+    return {k: torch.from_numpy(v.copy()).cuda() for k, v in p.items()}
+
+
+@pytest.mark.parametrize("n", [65535, 65536, 70001])
+@pytest.mark.parametrize("grid", [(1, 1, 1), (1, 1, 300), (17, 5, 9), (40, 24, 16)])
+@pytest.mark.parametrize("where", ["anywhere", "one cell", "nodes"])
+def test_against_oracle(cuda, n, grid, where):
+    torch = cuda
+    from sputnipic_b200 import device
+    rng = np.random.default_rng(n + grid[2])
+    wl = W.GemWorkload(name="t", nxc=grid[0], nyc=grid[1], nzc=grid[2], Lx=grid[0] * 0.3,
+                       Ly=grid[1] * 0.25, Lz=grid[2] * 0.7)
+    p = particles(rng, wl, n, where)
+    ctx = device.GridContext(wl)
+    mom = torch.zeros(10, wl.nodes, device="cuda")
+    ctx.p2g(on_gpu(torch, p), mom)
+    assert ctx.check() == 0
+    check(mom.cpu().numpy(), wl, p)
+    once = mom.clone()
+    ctx.p2g(on_gpu(torch, p), mom)   # a second call adds
+    assert torch.allclose(mom, 2 * once, rtol=1e-4, atol=1e-5 * float(once.abs().max()))
+    ctx.close()
+
+
+def test_shifted_domain_and_off_grid(cuda):
+    torch = cuda
+    from sputnipic_b200 import device, dropin
+    rng = np.random.default_rng(3)
+    wl = W.GemWorkload(name="t", nxc=12, nyc=10, nzc=7, Lx=3.0, Ly=2.5, Lz=1.75)   # cells of 0.25
+    n = 66000
+    p = particles(rng, wl, n, "anywhere")
+    for k in "xyz":   # multiples of 2^-18: shifting by 0.5 is exact
+        p[k] = (np.floor(p[k] * 2 ** 18) / 2 ** 18).astype(np.float32)
+    grd = dropin.setGrid(dropin.make_parameters(wl))
+    grd.xStart = grd.yStart = grd.zStart = 0.5
+    for a in ("XN", "YN", "ZN"):
+        grd._arrays[a] += np.float32(0.5)
+    ctx = device.GridContext(grid=grd)
+    mom = torch.zeros(10, wl.nodes, device="cuda")
+    moved = {k: (v + np.float32(0.5) if k in "xyz" else v) for k, v in p.items()}
+    ctx.p2g(on_gpu(torch, moved), mom)
+    assert ctx.check() == 0
+    check(mom.cpu().numpy(), wl, p)
+    ctx.close()
+    # positions off the node array are flagged and clamped, on both paths
+    from sputnipic_b200 import _lib
+    for shift in (0.0, 0.5):
+        ctx = device.GridContext(wl) if shift == 0.0 else device.GridContext(grid=grd)
+        for bad in (1e9, -1e9, float("nan")):
+            q = on_gpu(torch, p)
+            q["y"][5] = bad
+            ctx.p2g(q, mom)
+            with pytest.raises(_lib.SpbError):
+                _lib.check(ctx.check())
+        ctx.close()
+
+
+def test_more_than_one_chunk(cuda):
+    torch = cuda
+    from sputnipic_b200 import device
+    wl = W.GemWorkload(name="t", nxc=32, nyc=32, nzc=32, Lx=8.0, Ly=8.0, Lz=8.0)
+    n = (1 << 26) + 100_001
+    g = torch.Generator(device="cuda").manual_seed(1)
+    p = {k: torch.rand(n, generator=g, device="cuda") * (8.0 if k in "xyz" else 0.1) for k in "xyzuvwq"}
+    ctx = device.GridContext(wl)
+    whole = torch.zeros(10, wl.nodes, device="cuda")
+    ctx.p2g(p, whole)
+    parts = torch.zeros(10, wl.nodes, device="cuda")
+    for a, b in ((0, n // 3), (n // 3, n)):
+        ctx.p2g({k: v[a:b].contiguous() for k, v in p.items()}, parts)
+    assert ctx.check() == 0
+    # all terms positive: two FP32 sums of the same 2048 * 8 terms a node
+    assert float(((whole - parts).norm(dim=1) / whole.norm(dim=1)).max()) < 2e-6
+    ctx.close()
