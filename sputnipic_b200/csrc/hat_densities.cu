@@ -2,16 +2,17 @@
 // implicit sources of the field solver, J hat on the nodes and rho hat on the
 // cell centres, from the species moments, in the reference's arithmetic.
 //
-// Six launches for all species: the divergence of every species' pressure
+// Three launches for all species: the divergence of every species' pressure
 // tensor on the inner cells (divSymmTensorN2C, src/Grid.cpp:322-396) scaled by
-// -dt/2; the centre guard cells of all 3 ns temporaries (applyBCscalarDensC,
-// src/BC.cpp:623-727); one node pass that, species by species, interpolates
-// the centres to the inner nodes (interpC2Ninterp, src/Grid.cpp:122-139),
-// adds the species' J, rotates with its omega_c dt/2 and accumulates J hat
-// in registers (the PIdot loop, MaxwellSolver.cpp:535-566); the node guards
-// of J hat (applyBCscalarDensN, src/BC.cpp:11-121); one cell pass for
-// rho hat = rho_c - dt theta div(J hat) (divN2C, src/Grid.cpp:267-319); the
-// centre guards of rho hat.
+// -dt/2; one node pass that, species by species, interpolates the centres to
+// the nodes (interpC2Ninterp, src/Grid.cpp:122-139), adds the species' J,
+// rotates with its omega_c dt/2 and accumulates J hat in registers (the PIdot
+// loop, MaxwellSolver.cpp:535-566); one cell pass for rho hat = rho_c - dt
+// theta div(J hat) (divN2C, src/Grid.cpp:267-319). The guard cells that the
+// reference fills in between (applyBCscalarDensC, src/BC.cpp:623-727, of the
+// centre temporaries and of rho hat; applyBCscalarDensN, src/BC.cpp:11-121, of
+// J hat) each take the value of one inner cell (guard_source), so they are
+// read, or computed, where that cell is: no fill passes.
 //
 // Arithmetic. This file is compiled with -fmad=false and follows the C
 // promotions of the reference expressions: the stencils' .25 * (a - b) * inv
@@ -20,10 +21,6 @@
 // the array type. The float instantiation reproduces the reference's FP32
 // build bit for bit, the double one its FP64 build.
 //
-// Guard values. The reference leaves its temporaries' guard entries
-// uninitialised; the guard-cell fills overwrite every one of them before it
-// is read, each with the value its phase-by-phase fill would leave there
-// (fill_source).
 #include <algorithm>
 #include <cstring>
 
@@ -38,6 +35,7 @@ struct HatGeom {
   int nxc, nyc, nzc;   // cells, guard cells included
   int nxn, nyn, nzn;   // nodes
   double inv[3];       // the grid's inverse spacings
+  int per[3];          // periodic axes
 };
 
 __device__ __forceinline__ long nidx(const HatGeom &g, int i, int j, int k) {
@@ -90,145 +88,101 @@ struct Species6 {
   T beta[HAT_MAXS];
 };
 
+// The nodes (i; j, j + 1; k, k + 1) of the six pressure components.
+template <typename T>
+struct Plane6 {
+  T v[6][4];   // [component][2 (j + 1) + (k + 1)]
+};
+
+template <typename T>
+__device__ __forceinline__ void load_plane(const HatGeom &g, const T *const (&p)[6], long at,
+                                           Plane6<T> &P) {
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    P.v[c][0] = __ldg(p[c] + at);
+    P.v[c][1] = __ldg(p[c] + at + 1);
+    P.v[c][2] = __ldg(p[c] + at + g.nzn);
+    P.v[c][3] = __ldg(p[c] + at + g.nzn + 1);
+  }
+}
+
+// d4 of component c between the planes i (lo) and i + 1 (hi) along `axis`.
+template <typename T>
+__device__ __forceinline__ double d4_planes(const HatGeom &g, const Plane6<T> &lo,
+                                            const Plane6<T> &hi, int c, int axis) {
+  double sum = 0.0;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int a = t >> 1, b = t & 1;   // d4's hi and lo
+    T diff;
+    if (axis == 0)
+      diff = hi.v[c][2 * a + b] - lo.v[c][2 * a + b];
+    else if (axis == 1)
+      diff = (a ? hi : lo).v[c][2 + b] - (a ? hi : lo).v[c][b];
+    else
+      diff = (b ? hi : lo).v[c][2 * a + 1] - (b ? hi : lo).v[c][2 * a];
+    const double term = 0.25 * (double)diff * g.inv[axis];
+    sum = t ? sum + term : term;
+  }
+  return sum;
+}
+
 // Pressure-tensor rows (pxx pxy pxz / pxy pyy pyz / pxz pyz pzz): divergence
 // of each row on the inner cells, times alfa = (T)(-dt/2); species blockIdx.y.
-// Five CTAs per SM (at most 51 registers; a few bytes spill): the pass is
-// bound by the latency of its FP64 stencil loads, so residency pays.
+// A thread walks `run` cells along x and keeps the nodes of the last plane, so
+// a cell costs 24 loads (four nodes of six components) instead of the 72 that
+// its nine stencils read one by one: those kept the L1 pipe busy (an unaligned
+// row of 32 doubles takes three passes). 128x64x64 cells, 4 species, FP64: 62 ->
+// 46 us; with the guard fills gone the whole call 168 -> 110 us.
 template <typename T>
-__global__ void __launch_bounds__(256, 5) k_hat_div_tensor(HatGeom g, const __grid_constant__ Species6<T> S, T alfa) {
+__global__ void __launch_bounds__(128) k_hat_div_tensor(HatGeom g, const __grid_constant__ Species6<T> S, T alfa, int run) {
   const int is = blockIdx.y;
-  const int mx = g.nxc - 2, my = g.nyc - 2, mz = g.nzc - 2;
-  const long inner = (long)mx * my * mz;
-  // row r, column ax -> tensor component
-  const int comp[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < inner;
-       t += (long)gridDim.x * blockDim.x) {
-    const int k = 1 + (int)(t % mz), j = 1 + (int)((t / mz) % my), i = 1 + (int)(t / ((long)mz * my));
+  const int my = g.nyc - 2, mz = g.nzc - 2;
+  const unsigned columns = (unsigned)(((long)my * mz + 127) / 128);   // CTAs per run
+  const long t = (blockIdx.x % columns) * 128L + threadIdx.x;
+  if (t >= (long)my * mz) return;
+  const int k = 1 + (int)(t % mz), j = 1 + (int)(t / mz);
+  const int first = 1 + (int)(blockIdx.x / columns) * run, last = min(first + run, g.nxc - 1);
+  const T *const p[6] = {S.p[is][0], S.p[is][1], S.p[is][2], S.p[is][3], S.p[is][4], S.p[is][5]};
+  const long plane = (long)g.nyn * g.nzn;
+  long at = nidx(g, first, j, k), to = cidx(g, first, j, k);
+  auto cell = [&](const Plane6<T> &lo, const Plane6<T> &hi) {
+    // row r, column ax -> tensor component
+    const int comp[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-      const T c0 = (T)d4(g, S.p[is][comp[r][0]], i, j, k, 0);
-      const T c1 = (T)d4(g, S.p[is][comp[r][1]], i, j, k, 1);
-      const T c2 = (T)d4(g, S.p[is][comp[r][2]], i, j, k, 2);
+      const T c0 = (T)d4_planes(g, lo, hi, comp[r][0], 0);
+      const T c1 = (T)d4_planes(g, lo, hi, comp[r][1], 1);
+      const T c2 = (T)d4_planes(g, lo, hi, comp[r][2], 2);
       const T div = c0 + c1 + c2;
-      S.tc[is][r][cidx(g, i, j, k)] = div * alfa;
+      S.tc[is][r][to] = div * alfa;
+    }
+    to += (long)g.nyc * g.nzc;
+  };
+  Plane6<T> A, B;
+  load_plane(g, p, at, A);
+  for (int i = first; i < last; i += 2) {
+    load_plane(g, p, at += plane, B);
+    cell(A, B);
+    if (i + 1 < last) {
+      load_plane(g, p, at += plane, A);
+      cell(B, A);
     }
   }
 }
 
-// Guard-cell fill of n0 x n1 x n2 scalar arrays (applyBCscalarDensC with
-// s = 1, applyBCscalarDensN with s = 2). The reference's phases: periodic
-// faces X, Y, Z; edges along X, Y, Z; corners; non-periodic faces X, Y, Z. A
-// periodic face copies from n-1-s to 0 and from s to n-1; yhi ends the
-// Y-edge loop (nyn - 1 in both reference functions). Every guard cell gets
-// the value of one cell of the array before the fill (fill_source), so the
-// fill runs as one gather of all guard values and one scatter.
-struct Fill {
-  int n0, n1, n2, s, yhi;
-  int per[3];
-};
-
-template <typename T>
-struct Arrays {
-  T *a[3 * HAT_MAXS];
-};
-
-// The guard cells of an n0 x n1 x n2 array, numbered face by face: the two x
-// faces (every j, k), the two y faces (inner i, every k), the two z faces
-// (inner i, j).
-__host__ __device__ __forceinline__ long guard_count(const Fill &f) {
-  return 2L * f.n1 * f.n2 + 2L * (f.n0 - 2) * f.n2 + 2L * (f.n0 - 2) * (f.n1 - 2);
-}
-
-__device__ __forceinline__ void guard_cell(const Fill &f, long g, int &i, int &j, int &k) {
-  const long fx = (long)f.n1 * f.n2, fy = (long)(f.n0 - 2) * f.n2;
-  if (g < 2 * fx) {
-    i = g < fx ? 0 : f.n0 - 1;
-    const long r = g % fx;
-    j = (int)(r / f.n2);
-    k = (int)(r % f.n2);
-  } else if ((g -= 2 * fx) < 2 * fy) {
-    j = g < fy ? 0 : f.n1 - 1;
-    const long r = g % fy;
-    i = 1 + (int)(r / f.n2);
-    k = (int)(r % f.n2);
-  } else {
-    g -= 2 * fy;
-    const long fz = (long)(f.n0 - 2) * (f.n1 - 2);
-    k = g < fz ? 0 : f.n2 - 1;
-    const long r = g % fz;
-    i = 1 + (int)(r / (f.n1 - 2));
-    j = 1 + (int)(r % (f.n1 - 2));
-  }
-}
-
-// Periodic source along one axis: the guard at e copies from s, the guard
-// at 0 from e - s.
-__device__ __forceinline__ int per_src(int x, int e, int s) {
-  return x == e ? s : (x == 0 ? e - s : x);
-}
-
-// The cell whose value before the fill ends up in cell (i, j, k) after it
-// (every phase of the reference's fill copies one cell into another and
-// never writes what it reads). The phases in the reference order are:
-// periodic faces X, Y, Z; edges along X, Y (j < yhi only), Z; corners;
-// non-periodic faces X, Y, Z. Walking them backwards, each phase that writes
-// the current cell replaces it by that phase's source.
-__device__ __forceinline__ void fill_source(const Fill &f, int &i, int &j, int &k) {
-  const int e0 = f.n0 - 1, e1 = f.n1 - 1, e2 = f.n2 - 1, s = f.s;
-  const bool p0 = f.per[0], p1 = f.per[1], p2 = f.per[2];
-  auto guard = [](int x, int e) { return x == 0 || x == e; };
-  auto inner = [](int x, int e) { return x >= 1 && x <= e - 1; };
-  if (!p2 && guard(k, e2)) k = k == 0 ? 1 : e2 - 1;   // non-periodic Z faces
-  if (!p1 && guard(j, e1)) j = j == 0 ? 1 : e1 - 1;   // non-periodic Y faces
-  if (!p0 && guard(i, e0)) i = i == 0 ? 1 : e0 - 1;   // non-periodic X faces
-  if ((p0 || p1 || p2) && guard(i, e0) && guard(j, e1) && guard(k, e2)) {   // corners
-    i = per_src(i, e0, s);
-    j = per_src(j, e1, s);
-    k = per_src(k, e2, s);
-  }
-  if ((p0 || p1) && inner(k, e2) && guard(i, e0) && guard(j, e1)) {   // edges along Z
-    i = per_src(i, e0, s);
-    j = per_src(j, e1, s);
-  }
-  if ((p0 || p2) && j >= 1 && j <= f.yhi - 1 && guard(i, e0) && guard(k, e2)) {   // along Y
-    i = per_src(i, e0, s);
-    k = per_src(k, e2, s);
-  }
-  if ((p1 || p2) && inner(i, e0) && guard(j, e1) && guard(k, e2)) {   // edges along X
-    j = per_src(j, e1, s);
-    k = per_src(k, e2, s);
-  }
-  if (p2 && inner(i, e0) && inner(j, e1) && guard(k, e2)) k = per_src(k, e2, s);   // Z faces
-  if (p1 && inner(i, e0) && inner(k, e2) && guard(j, e1)) j = per_src(j, e1, s);   // Y faces
-  if (p0 && inner(j, e1) && inner(k, e2) && guard(i, e0)) i = per_src(i, e0, s);   // X faces
-}
-
-// Guard-cell fill of narr arrays, first pass: every guard cell's final value
-// (from its fill_source, before any guard cell changes) into tmp.
-template <typename T>
-__global__ void k_hat_guard_gather(Fill f, const __grid_constant__ Arrays<T> A, int narr,
-                                   T *__restrict__ tmp) {
-  const long G = guard_count(f), total = narr * G;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total;
-       t += (long)gridDim.x * blockDim.x) {
-    int i, j, k;
-    guard_cell(f, t % G, i, j, k);
-    fill_source(f, i, j, k);
-    tmp[t] = A.a[t / G][((long)i * f.n1 + j) * f.n2 + k];
-  }
-}
-
-// Second pass: the values into the guard cells.
-template <typename T>
-__global__ void k_hat_guard_scatter(Fill f, const __grid_constant__ Arrays<T> A, int narr,
-                                    const T *__restrict__ tmp) {
-  const long G = guard_count(f), total = narr * G;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total;
-       t += (long)gridDim.x * blockDim.x) {
-    int i, j, k;
-    guard_cell(f, t % G, i, j, k);
-    A.a[t / G][((long)i * f.n1 + j) * f.n2 + k] = tmp[t];
-  }
+// The inner cell whose value a cell holds after the reference's guard-cell
+// fill, per axis: x itself inside; on a periodic axis of n cells the guard at 0
+// holds cell n - 1 - s and the one at n - 1 cell s (s = 1 for centres, 2 for
+// nodes), on another axis the neighbouring cell. The reference fills in phases
+// (periodic faces X, Y, Z; edges; corners; the other faces X, Y, Z), each of
+// which copies cells by these rules axis by axis; the phases' combined effect
+// on a guard cell of several axes is the axes' rules one by one.
+__device__ __forceinline__ int guard_source(int x, int n, int s, int periodic) {
+  const int e = n - 1;
+  if (x == 0) return periodic ? e - s : 1;
+  if (x == e) return periodic ? s : e - 1;
+  return x;
 }
 
 template <typename T>
@@ -240,37 +194,43 @@ struct Out3 {
   T *v[3];
 };
 
-// Every node: per species in order, the interpolated divergence (inner
-// nodes) plus J, rotated by the species' beta B and added into J hat, which
-// starts at 0 (the reference's per-species accumulation, in registers).
-// Four CTAs per SM (at most 64 registers), for the same reason.
+// Every node: per species in order, the interpolated divergence plus J,
+// rotated by the species' beta B and added into J hat, which starts at 0 (the
+// reference's per-species accumulation, in registers). A guard node computes
+// the node that its value comes from, and guard cells are read where theirs
+// does. Four CTAs per SM (at most 64 registers), for the same reason.
 template <typename T>
 __global__ void __launch_bounds__(256, 4) k_hat_pidot(HatGeom g, const __grid_constant__ Species6<T> S, int ns, Vec3<T> B,
                             Out3<T> JH) {
   const long nodes = (long)g.nxn * g.nyn * g.nzn;
   for (long n = blockIdx.x * (long)blockDim.x + threadIdx.x; n < nodes;
        n += (long)gridDim.x * blockDim.x) {
-    const int k = (int)(n % g.nzn), j = (int)((n / g.nzn) % g.nyn), i = (int)(n / ((long)g.nzn * g.nyn));
-    const bool inner = i >= 1 && i < g.nxn - 1 && j >= 1 && j < g.nyn - 1 && k >= 1 && k < g.nzn - 1;
-    const T bx = B.v[0][n], by = B.v[1][n], bz = B.v[2][n];
+    const int i = guard_source((int)(n / ((long)g.nzn * g.nyn)), g.nxn, 2, g.per[0]);
+    const int j = guard_source((int)((n / g.nzn) % g.nyn), g.nyn, 2, g.per[1]);
+    const int k = guard_source((int)(n % g.nzn), g.nzn, 2, g.per[2]);
+    const long m = nidx(g, i, j, k);
+    // the node's upper cell, and the steps to its lower ones per axis
+    const int i0 = guard_source(i, g.nxc, 1, g.per[0]), j0 = guard_source(j, g.nyc, 1, g.per[1]),
+              k0 = guard_source(k, g.nzc, 1, g.per[2]);
+    const long c0 = cidx(g, i0, j0, k0);
+    const long dx = (long)(guard_source(i - 1, g.nxc, 1, g.per[0]) - i0) * g.nyc * g.nzc;
+    const int dy = (guard_source(j - 1, g.nyc, 1, g.per[1]) - j0) * g.nzc;
+    const int dz = guard_source(k - 1, g.nzc, 1, g.per[2]) - k0;
+    const T bx = B.v[0][m], by = B.v[1][m], bz = B.v[2][m];
     T jh[3] = {(T)0, (T)0, (T)0};
     for (int is = 0; is < ns; ++is) {
       T tn[3];
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        T v = (T)0;
-        if (inner) {
-          const T *c = S.tc[is][r];
-          T s8 = c[cidx(g, i, j, k)] + c[cidx(g, i - 1, j, k)];
-          s8 = s8 + c[cidx(g, i, j - 1, k)];
-          s8 = s8 + c[cidx(g, i, j, k - 1)];
-          s8 = s8 + c[cidx(g, i - 1, j - 1, k)];
-          s8 = s8 + c[cidx(g, i - 1, j, k - 1)];
-          s8 = s8 + c[cidx(g, i, j - 1, k - 1)];
-          s8 = s8 + c[cidx(g, i - 1, j - 1, k - 1)];
-          v = (T)(0.125 * (double)s8);
-        }
-        tn[r] = v + S.j[is][r][n];
+        const T *c = S.tc[is][r] + c0;
+        T s8 = c[0] + c[dx];
+        s8 = s8 + c[dy];
+        s8 = s8 + c[dz];
+        s8 = s8 + c[dx + dy];
+        s8 = s8 + c[dx + dz];
+        s8 = s8 + c[dy + dz];
+        s8 = s8 + c[dx + dy + dz];
+        tn[r] = (T)(0.125 * (double)s8) + S.j[is][r][m];
       }
       const T beta = S.beta[is];
       const T ox = beta * bx, oy = beta * by, oz = beta * bz;
@@ -288,23 +248,22 @@ __global__ void __launch_bounds__(256, 4) k_hat_pidot(HatGeom g, const __grid_co
   }
 }
 
-// rho hat = rho_c - dt theta div(J hat) on every cell (the divergence is 0 on
-// the guard cells, whose values the final fill replaces).
+// rho hat = rho_c - dt theta div(J hat) on every cell; a guard cell computes
+// the cell that its value comes from.
 template <typename T>
 __global__ void k_hat_rho(HatGeom g, Vec3<T> JH, const T *__restrict__ rhoc, double dt_th,
                           T *__restrict__ rhoh) {
   const long cells = (long)g.nxc * g.nyc * g.nzc;
   for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < cells;
        c += (long)gridDim.x * blockDim.x) {
-    const int k = (int)(c % g.nzc), j = (int)((c / g.nzc) % g.nyc), i = (int)(c / ((long)g.nzc * g.nyc));
-    T dv = (T)0;
-    if (i >= 1 && i < g.nxc - 1 && j >= 1 && j < g.nyc - 1 && k >= 1 && k < g.nzc - 1) {
-      const T cx = (T)d4(g, JH.v[0], i, j, k, 0);
-      const T cy = (T)d4(g, JH.v[1], i, j, k, 1);
-      const T cz = (T)d4(g, JH.v[2], i, j, k, 2);
-      dv = cx + cy + cz;
-    }
-    rhoh[c] = (T)((double)rhoc[c] - dt_th * (double)dv);
+    const int i = guard_source((int)(c / ((long)g.nzc * g.nyc)), g.nxc, 1, g.per[0]);
+    const int j = guard_source((int)((c / g.nzc) % g.nyc), g.nyc, 1, g.per[1]);
+    const int k = guard_source((int)(c % g.nzc), g.nzc, 1, g.per[2]);
+    const T cx = (T)d4(g, JH.v[0], i, j, k, 0);
+    const T cy = (T)d4(g, JH.v[1], i, j, k, 1);
+    const T cz = (T)d4(g, JH.v[2], i, j, k, 2);
+    const T dv = cx + cy + cz;
+    rhoh[c] = (T)((double)rhoc[cidx(g, i, j, k)] - dt_th * (double)dv);
   }
 }
 
@@ -331,55 +290,38 @@ int hat_densities(const spb_hat_desc *d, const T *const *mom, const T *const B[3
   g.inv[0] = d->invdx;
   g.inv[1] = d->invdy;
   g.inv[2] = d->invdz;
+  for (int a = 0; a < 3; ++a) g.per[a] = d->periodic[a] ? 1 : 0;
   const long cells = (long)g.nxc * g.nyc * g.nzc, nodes = (long)g.nxn * g.nyn * g.nzn;
   const int ns = d->ns;
-  Fill fc{g.nxc, g.nyc, g.nzc, 1, g.nyn - 1, {d->periodic[0], d->periodic[1], d->periodic[2]}};
-  Fill fn{g.nxn, g.nyn, g.nzn, 2, g.nyn - 1, {d->periodic[0], d->periodic[1], d->periodic[2]}};
-  // three centre temporaries per species, then the guard fills' buffer
-  const long gtmp = std::max(3 * ns * guard_count(fc), 3 * guard_count(fn));
+  // three centre temporaries per species (their guard cells are never written)
   T *tc = nullptr;
-  SPB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&tc),
-                           (3 * ns * cells + gtmp) * sizeof(T), st));
-  T *const gbuf = tc + 3 * ns * cells;
-  auto fill = [&](const Fill &f, const Arrays<T> &arr, int narr) {
-    const unsigned blocks = (unsigned)std::min<long>(blocks_for(narr * guard_count(f), 256), 4096);
-    k_hat_guard_gather<T><<<blocks, 256, 0, st>>>(f, arr, narr, gbuf);
-    k_hat_guard_scatter<T><<<blocks, 256, 0, st>>>(f, arr, narr, gbuf);
-  };
+  SPB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&tc), 3 * ns * cells * sizeof(T), st));
   Species6<T> S;   // kernel parameters (copied at launch)
-  Arrays<T> A;
   std::memset(&S, 0, sizeof(S));
-  std::memset(&A, 0, sizeof(A));
   for (int is = 0; is < ns; ++is) {
     const T *const *M = mom + 10 * is;
     for (int c = 0; c < 6; ++c) S.p[is][c] = M[4 + c];
     for (int r = 0; r < 3; ++r) {
       S.j[is][r] = M[1 + r];
       S.tc[is][r] = tc + (3 * is + r) * cells;
-      A.a[3 * is + r] = S.tc[is][r];
     }
     S.beta[is] = (T)(.5 * d->qom[is] * d->dt / d->c);
   }
   const T alfa = (T)(-d->dt / 2.0);
   const long inner = (long)(g.nxc - 2) * (g.nyc - 2) * (g.nzc - 2);
   int rc = SPB_OK;
-  const int gx = std::max(1, blocks_for(inner, 256) / ns);
-  k_hat_div_tensor<T><<<dim3(gx, ns), 256, 0, st>>>(g, S, alfa);
-  fill(fc, A, 3 * ns);
+  // cells per thread along x: eight, fewer where that would leave SMs without
+  // a full set of threads
+  const int run = (int)std::max(1L, std::min(8L, inner * ns / (148L * 512)));
+  const dim3 grid((unsigned)(ceil_div((long)(g.nyc - 2) * (g.nzc - 2), 128) *
+                             ceil_div(g.nxc - 2, run)), (unsigned)ns);
+  k_hat_div_tensor<T><<<grid, 128, 0, st>>>(g, S, alfa, run);
   k_hat_pidot<T><<<blocks_for(nodes, 256), 256, 0, st>>>(g, S, ns, Vec3<T>{{B[0], B[1], B[2]}},
                                                          Out3<T>{{jxh, jyh, jzh}});
-  Arrays<T> J{};
-  J.a[0] = jxh;
-  J.a[1] = jyh;
-  J.a[2] = jzh;
-  fill(fn, J, 3);
   k_hat_rho<T><<<blocks_for(cells, 256), 256, 0, st>>>(g, Vec3<T>{{jxh, jyh, jzh}}, rhoc,
                                                        d->dt * d->th, rhoh);
-  Arrays<T> R{};
-  R.a[0] = rhoh;
-  fill(fc, R, 1);
   if (cudaGetLastError() != cudaSuccess) rc = fail(SPB_ERR_CUDA, "spb_hat_densities: launch");
-  g_launches += 9;
+  g_launches += 3;
   cudaFreeAsync(tc, st);
   return rc;
 }
