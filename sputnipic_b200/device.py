@@ -26,6 +26,17 @@ def _ptr(t) -> int:
     return t.data_ptr()
 
 
+def _mom_ptrs(mom):
+    """Addresses of the ten moment arrays mom[0..9]: of one contiguous tensor from its own address
+    and stride (slicing it ten times costs more than a small deposit's kernels), else one by one."""
+    import torch
+    if (isinstance(mom, torch.Tensor) and mom.dim() >= 2 and mom.shape[0] >= 10 and mom.is_cuda
+            and mom.dtype == torch.float32 and mom.is_contiguous()):
+        p, step = mom.data_ptr(), 4 * mom.stride(0)
+        return (ctypes.c_void_p * 10)(*[p + i * step for i in range(10)])
+    return (ctypes.c_void_p * 10)(*[_ptr(mom[i]) for i in range(10)])
+
+
 DEPOSIT_MODES = {"accumulator": 0, "direct": 1}
 
 
@@ -96,20 +107,20 @@ class GridContext:
 
     def p2g(self, part, mom, stream=None):
         n = part["x"].numel()
-        m = (ctypes.c_void_p * 10)(*[_ptr(mom[i]) for i in range(10)])
+        m = _mom_ptrs(mom)
         _lib.check(self.lib.spb_grid_p2g(self.h, *[_ptr(part[k]) for k in "xyzuvwq"], n, m,
                                          _stream(stream)))
 
     def mover_interp(self, part, push, mom, stream=None):
         n = part["x"].numel()
-        m = (ctypes.c_void_p * 10)(*[_ptr(mom[i]) for i in range(10)])
+        m = _mom_ptrs(mom)
         _lib.check(self.lib.spb_grid_mover_interp(self.h, ctypes.byref(push),
                                                   *[_ptr(part[k]) for k in "xyzuvwq"], n, m,
                                                   _stream(stream)))
 
     def apply_bc_ids(self, mom, periodic, stream=None):
         per = (ctypes.c_int * 3)(*[1 if p else 0 for p in periodic])
-        m = (ctypes.c_void_p * 10)(*[_ptr(mom[i]) for i in range(10)])
+        m = _mom_ptrs(mom)
         _lib.check(self.lib.spb_grid_apply_bc_ids(self.h, ctypes.byref(per), m, _stream(stream)))
 
     def check(self, stream=None) -> int:
