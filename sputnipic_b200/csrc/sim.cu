@@ -62,18 +62,6 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
                : "memory");
 }
 
-// Raises the barrier's expected transaction bytes without arriving: several
-// copies can be armed one by one and the phase closed by one mbar_arrive.
-__device__ __forceinline__ void mbar_expect_tx_only(uint64_t *bar, unsigned bytes) {
-  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned phase) {
   unsigned ok;
   asm volatile(
@@ -106,17 +94,6 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, i
 
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// Untiled bulk copy global -> this CTA's shared memory (no multicast),
-// completion on `bar`. Both addresses 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes,
-                                          uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_addr(dst)),
-      "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_addr(bar))
-      : "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -215,9 +192,13 @@ struct Tile {
   static constexpr int BX = TX + 3, BY = TY + 3, BZ = TZ + 3;
   static constexpr int BN = BX * BY * BZ;    // staged nodes
   static constexpr int TC = TX * TY * TZ;    // cells per tile
-  // floats per field stage, padded so every stage starts on the 128-byte
-  // boundary a TMA tensor copy's shared-memory destination needs
-  static constexpr int SF = ((8 * BN + 31) / 32) * 32;
+  // floats per field stage: (Ex, Ey, Ez, Bx) of every node, then (By, Bz, -, -)
+  // of every node from float SH on, each part padded so that it starts on the
+  // 128-byte boundary a TMA tensor copy's shared-memory destination needs. Two
+  // parts of 16 bytes per node, not one of 32: eight neighbouring nodes then
+  // fall in eight different bank groups of a 128-bit load instead of four.
+  static constexpr int SH = ((4 * BN + 31) / 32) * 32;
+  static constexpr int SF = 2 * SH;
   static_assert((SF * 4) % 128 == 0, "field stages must stay 128-byte aligned");
 };
 
@@ -271,8 +252,8 @@ __device__ __forceinline__ Field6 gather(const float *__restrict__ sF, int n0, f
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const int n = n0 + (a * T::BY + b) * T::BZ + c;
-        const float4 A = *reinterpret_cast<const float4 *>(sF + 8 * n);
-        const float2 B = *reinterpret_cast<const float2 *>(sF + 8 * n + 4);
+        const float4 A = *reinterpret_cast<const float4 *>(sF + 4 * n);
+        const float2 B = *reinterpret_cast<const float2 *>(sF + T::SH + 4 * n);
         if (b == 0 && c == 0)   // each layer's sum starts from its first product
           F[a] = first_node(__fmul_rn(wab, wz[c]), A, B);
         else
@@ -398,13 +379,21 @@ __device__ __forceinline__ void push(const CycleParams &P, const float *__restri
   }
 }
 
-// Stores one pushed record in slot `slot` of the bucket [dbase, dend) of cell
+// Read-only 32-byte load of one particle record of a slot (neighbouring lanes
+// read neighbouring records, so nothing is asked of L2 beyond them).
+__device__ __forceinline__ void ld_slot(const float4 *p, float4 &a, float4 &b) {
+  asm("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
+// Stores one pushed record in slot `slot` of the `cap` slots from dbase of cell
 // `key`, or appends it to the overflow list when the bucket is full. Returns
 // 1 if the overflow list was full too (the particle is lost; reported).
 
-__device__ __forceinline__ int put_at(const SpeciesDev &S, int key, long long dbase,
-                                      long long dend, int slot, float4 a, float4 b) {
-  if (dbase + slot < dend) {
+__device__ __forceinline__ int put_at(const SpeciesDev &S, int key, long long dbase, int cap,
+                                      int slot, float4 a, float4 b) {
+  if (slot < cap) {
     st_rec(S.rout + 2 * (dbase + slot), a, b);
     return 0;
   }
@@ -422,19 +411,19 @@ __device__ __forceinline__ int put_at(const SpeciesDev &S, int key, long long db
 // one atomic. The records wait in a per-warp shared-memory staging area (two
 // float4 per lane).
 struct Pending {
-  long long dbase, dend;  // destination bucket
+  long long dbase;        // destination bucket: first slot,
+  int cap;                // and slots (0: the overflow list whatever its room)
   int key;                // destination cell
   int slot0;              // group leader: first slot reserved for its group
-  int leader, rank;       // this lane's group leader and rank in the group
-  bool valid;
+  int group;              // this lane's group leader, its rank in the group << 8; < 0: no particle
 };
 
 // Completes a pending slot. All 32 lanes call.
 __device__ __forceinline__ void flush(const SpeciesDev &S, const Pending &p, const float4 *stage,
                                       int lane, int &lost) {
-  const int s0 = __shfl_sync(FULL, p.slot0, p.leader);
-  if (p.valid)
-    lost |= put_at(S, p.key, p.dbase, p.dend, s0 + p.rank, stage[lane], stage[32 + lane]);
+  const int s0 = __shfl_sync(FULL, p.slot0, p.group & 31);
+  if (p.group >= 0)
+    lost |= put_at(S, p.key, p.dbase, p.cap, s0 + (p.group >> 8), stage[lane], stage[32 + lane]);
 }
 
 // Issues the counter updates of a pushed slot and stages its records. All 32
@@ -446,24 +435,16 @@ __device__ __forceinline__ void issue_slot(const SpeciesDev &S, Pending &p, floa
                                           int nkey, bool valid, float4 a, float4 b, int lane,
                                           bool far = false) {
   const unsigned peers = __match_any_sync(FULL, valid ? nkey : -1);
-  p.leader = __ffs(peers) - 1;
-  p.rank = __popc(peers & ((1u << lane) - 1u));
+  const int leader = __ffs(peers) - 1;
+  p.group = valid ? leader | (__popc(peers & ((1u << lane) - 1u)) << 8) : (int)0x80000000;
   p.slot0 = 0;
   const bool place = valid && !far;
-  if (place && lane == p.leader) p.slot0 = atomicAdd(S.cout + nkey, __popc(peers));
+  if (place && lane == leader) p.slot0 = atomicAdd(S.cout + nkey, __popc(peers));
   p.key = nkey;
-  p.valid = valid;
   p.dbase = place ? __ldg(S.base + nkey) : 0;
-  p.dend = place ? __ldg(S.base + nkey + 1) : 0;
+  p.cap = place ? (int)(__ldg(S.base + nkey + 1) - p.dbase) : 0;
   stage[lane] = a;
   stage[32 + lane] = b;
-}
-
-// Records per half of a warp's record ring: 4 KB at two resident CTAs per SM,
-// 2 KB at three or more (so that three CTAs fit in shared memory).
-template <int MINB>
-__host__ __device__ constexpr int ring_half() {
-  return MINB >= 3 ? 64 : 128;
 }
 
 // Independent jobs (own grid, fields, species and buckets; one tile shape)
@@ -528,10 +509,6 @@ __device__ __forceinline__ void load_params(CycleParams *dst, const CycleParams 
 // Per-warp state of the push that lives across tiles and jobs.
 struct PushWarp {
   float4 *wrec;        // staged records of the pending slot
-  float4 *ring;        // record ring: two halves of RH records
-  uint64_t *cbar;      // the halves' barriers
-  unsigned phase = 0, inflight = 0;   // per half: next parity, copies armed
-  bool dead = false;   // a bounded wait for records ran out
   int bad = 0, lost = 0;
 };
 
@@ -540,10 +517,14 @@ struct PushWarp {
 //
 // Each warp owns NC cells of the tile (tile-local warp + j * NW) and pushes
 // their records as one stream: slot k holds the stream's records 32k..32k+31
-// whatever their cells, so slots stay full however the counts fall. Lane 0
-// copies the cells' records into a two-half ring (bulk copies, one per cell
-// piece; a half's barrier closes after its last piece is armed); a half is
-// refilled as soon as its last slot has been read.
+// whatever their cells, so slots stay full however the counts fall. A lane
+// loads its record of the next slot before it pushes this one's, one 256-bit
+// load that is back long before it is used (a slot takes a few thousand
+// cycles with the SM's other warps). Bulk copies of the cells' pieces into a
+// ring in shared memory, which these loads replace, cost an instruction stream
+// of their own per cell, waits, and 24 of the 160 passes through the shared-
+// memory pipe per slot. GEM grid, 4 species: 7021 -> 6239 us at 125 particles per
+// cell, 1735 -> 1479 us at 27, 691 -> 532 us at 8.
 // Whether a destination tile coordinate d tiles away on an axis of n tiles
 // (periodic or not) lies outside the source tile's neighbourhood.
 __device__ __forceinline__ bool far_axis(int d, int n, int periodic) {
@@ -551,12 +532,12 @@ __device__ __forceinline__ bool far_axis(int d, int n, int periodic) {
   return d < -1 || d > 1;
 }
 
-template <int TX, int TY, int TZ, int RH, bool FUSED = false>
+template <int TX, int TY, int TZ, bool FUSED = false>
 __device__ __forceinline__ void push_tile(const CycleParams &P, int tile, int s0, int s1,
                                           const float *sF, PushWarp &W) {
   using T = Tile<TX, TY, TZ>;
   constexpr int NC = T::TC / SIM_NW;   // cells per warp and tile
-  static_assert(RH % 32 == 0, "slots must not straddle ring halves");
+  static_assert((NC & (NC - 1)) == 0, "a power of two of cells per warp");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tz = tile % P.ntz, ty = (tile / P.ntz) % P.nty, tx = tile / (P.ntz * P.nty);
   const int c0x = tx * TX, c0y = ty * TY, c0z = tz * TZ;
@@ -579,67 +560,37 @@ __device__ __forceinline__ void push_tile(const CycleParams &P, int tile, int s0
     }
     const int total = __shfl_sync(FULL, cp, 31);
     cp -= cc;
-    if (total == 0 || W.dead) continue;
+    if (total == 0) continue;
 
-    int pj = 0, poff = 0, pv = 0;   // next record to copy: cell, offset, stream index
-    // Copies the next records (at most RH) into half h; all lanes call.
-    auto fill = [&](int h) {
-      const int end = min(pv + RH, total);
-      if (lane == 0) fence_proxy_async();   // the half's previous reads come first
-      while (pv < end) {
-        int cnt = __shfl_sync(FULL, cc, pj);
-        while (poff >= cnt && pj < NC - 1) {
-          ++pj;
-          poff = 0;
-          cnt = __shfl_sync(FULL, cc, pj);
-        }
-        const int n = min(cnt - poff, end - pv);
-        if (n <= 0) break;   // unreachable: the counts sum to total
-        const long long b0 = __shfl_sync(FULL, cb, pj);
-        if (lane == 0) {
-          mbar_expect_tx_only(W.cbar + h, (unsigned)n * 32u);
-          bulk_load(W.ring + 2 * (pv % (2 * RH)), S.rin + 2 * (b0 + poff), (unsigned)n * 32u,
-                    W.cbar + h);
-        }
-        pv += n;
-        poff += n;
+    // the lane's cell and record of the slot from stream index rv on; idle
+    // lanes of the last slot push a copy of the stream's last particle (results
+    // discarded): one instruction stream per warp. The cell is the last j with
+    // cp_j <= the lane's stream index.
+    auto load_slot = [&](int rv, int &j, float4 &a, float4 &b) {
+      const int ii = min(rv + lane, total - 1);
+      j = 0;
+#pragma unroll
+      for (int st = NC / 2; st > 0; st >>= 1) {
+        const int pc = __shfl_sync(FULL, cp, j + st);
+        if (pc <= ii) j += st;
       }
-      if (lane == 0) mbar_arrive(W.cbar + h);
-      W.inflight |= 1u << h;
+      const long long b0 = __shfl_sync(FULL, cb, j);
+      const int first = __shfl_sync(FULL, cp, j);
+      ld_slot(S.rin + 2 * (b0 + (ii - first)), a, b);
     };
-    fill(0);
-    if (pv < total) fill(1);
+    int j1;
+    float4 a1, b1;
+    load_slot(0, j1, a1, b1);
 
     Pending pend;
-    pend.valid = false;
-    pend.slot0 = pend.leader = pend.rank = 0;
+    pend.group = (int)0x80000000;
+    pend.slot0 = 0;
 #pragma unroll 1
     for (int rv = 0; rv < total; rv += 32) {
-      const int h = (rv / RH) & 1;
-      if (rv % RH == 0) {   // first slot of half h: wait for its copies
-        const bool ok = mbar_wait_bounded(W.cbar + h, (W.phase >> h) & 1u);
-        if (!__all_sync(FULL, ok)) {
-          W.dead = true;
-          break;
-        }
-        W.phase ^= 1u << h;
-        W.inflight &= ~(1u << h);
-      }
-      const int i = rv + lane;
-      const bool valid = i < total;
-      // idle lanes of the last slot push a copy of the stream's last particle
-      // (results discarded): one instruction stream per warp
-      const int ii = valid ? i : total - 1;
-      const float4 *rp = W.ring + 2 * (ii % (2 * RH));
-      const float4 a = rp[0], b = rp[1];
-      // the lane's cell: the last j with cp_j <= ii
-      int j = 0;
-#pragma unroll
-      for (int st = 16; st > 0; st >>= 1) {
-        const int cand = j + st;
-        const int pc = __shfl_sync(FULL, cp, cand & 31);
-        if (cand < NC && pc <= ii) j = cand;
-      }
+      const int j = j1;
+      const float4 a = a1, b = b1;
+      if (rv + 32 < total) load_slot(rv + 32, j1, a1, b1);
+      const bool valid = rv + lane < total;
       const int lc = warp + j * SIM_NW;
       const int lx = lc / (TY * TZ), ly = (lc / TZ) % TY, lz = lc % TZ;
       const int n0c = ((lx + 1) * T::BY + (ly + 1)) * T::BZ + (lz + 1);
@@ -659,11 +610,6 @@ __device__ __forceinline__ void push_tile(const CycleParams &P, int tile, int s0
       __syncwarp();
       issue_slot(S, pend, W.wrec, nkey, valid, make_float4(ox, oy, oz, a.w),
                  make_float4(u, v, w, 0.f), lane, far);
-      // last slot of half h read by every lane: refill it
-      if ((rv + 32) % RH == 0 && pv < total) {
-        __syncwarp();
-        fill(h);
-      }
     }
     flush(S, pend, W.wrec, lane, W.lost);
     __syncwarp();
@@ -703,7 +649,8 @@ __device__ __forceinline__ void push_overflow(const CycleParams &P, const float 
                            make_float4(u, v, w, 0.f));
         } else {
           const int slot = atomicAdd(S.cout + nkey, 1);
-          W.lost |= put_at(S, nkey, S.base[nkey], S.base[nkey + 1], slot,
+          const long long d0 = S.base[nkey];
+          W.lost |= put_at(S, nkey, d0, (int)(S.base[nkey + 1] - d0), slot,
                            make_float4(ox, oy, oz, a.w), make_float4(u, v, w, 0.f));
         }
       }
@@ -722,8 +669,8 @@ __device__ __forceinline__ void report(const CycleParams &P, PushWarp &W) {
 // CTAs walk tiles of TX x TY x TZ cells; one thread stages the tile's E/B
 // nodes plus a one-cell halo into shared memory with a TMA tensor copy (two
 // stages: the next tile's copy overlaps this tile's work). Warps walk the
-// tile's cells, one particle per lane, with the cells' records streamed
-// through two shared-memory chunk buffers per warp by bulk copies; the
+// tile's cells, one particle per lane, each lane loading its record of the
+// next slot before it pushes this one's; the
 // gathers of the NiterMover iterations read the staged tile (or L2 past the
 // halo), and every pushed particle is written into the bucket of its new
 // cell. Afterwards the CTAs push the overflow entries (gathers from L2).
@@ -734,21 +681,17 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
     k_push(const __grid_constant__ CUtensorMap fmap, const __grid_constant__ CycleParams P1,
            const __grid_constant__ JobTable J, const __grid_constant__ MapsOf<MULTI> M) {
   using T = Tile<TX, TY, TZ>;
-  constexpr int RH = ring_half<MINB>();
   static_assert(T::TC % SIM_NW == 0 && T::TC / SIM_NW <= 32,
                 "cells per warp must fit a warp's lanes");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float *sF0 = reinterpret_cast<float *>(smem_raw);                 // 2 stages x SF
   float4 *sRec = reinterpret_cast<float4 *>(sF0 + 2 * T::SF);       // NW x 64 staged records
-  float4 *sBuf = sRec + SIM_NW * 64;                                // NW x 2 x RH records
-  CycleParams *sP = reinterpret_cast<CycleParams *>(sBuf + SIM_NW * 2 * RH * 2);  // MULTI
-  uint64_t *bar = reinterpret_cast<uint64_t *>(sP + (MULTI ? 1 : 0));   // 2 + 2 NW
+  CycleParams *sP = reinterpret_cast<CycleParams *>(sRec + SIM_NW * 64);   // MULTI
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sP + (MULTI ? 1 : 0));   // 2
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5;
   PushWarp W;
   W.wrec = sRec + warp * 64;
-  W.ring = sBuf + warp * 2 * RH * 2;
-  W.cbar = bar + 2 + warp * 2;
   int *const err0 = MULTI ? J.params[0].err : P1.err;
   if (smem_addr(sF0) & 127u) {   // TMA destinations need 128-byte alignment
     if (tid == 0) atomicOr(err0, ERRBIT_SMEM_ALIGN);
@@ -757,10 +700,6 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
   if (tid == 0) {
     mbar_init(bar, 1);
     mbar_init(bar + 1, 1);
-  }
-  if (lane == 0) {
-    mbar_init(W.cbar, 1);
-    mbar_init(W.cbar + 1, 1);
   }
   __syncthreads();
 
@@ -791,6 +730,7 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
     mbar_expect_tx(bar + stage, box_bytes);
     // box origin: node c0 on every axis (the lower node of halo cell c0-1)
     tma_load_4d(sF0 + stage * T::SF, map, 0, z * TZ, y * TY, x * TX, bar + stage);
+    tma_load_4d(sF0 + stage * T::SF + T::SH, map, 4, z * TZ, y * TY, x * TX, bar + stage);
   };
   if (tid == 0 && blockIdx.x < ntiles) issue(blockIdx.x, 0);
   int it = 0, cur_job = -1;
@@ -816,23 +756,14 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
         load_params(sP, J.params + job);
         cur_job = job;
       }
-      push_tile<TX, TY, TZ, RH>(*sP, local, s0, s1, sF, W);
+      push_tile<TX, TY, TZ>(*sP, local, s0, s1, sF, W);
       report(*sP, W);
     } else {
-      push_tile<TX, TY, TZ, RH>(P1, local, s0, s1, sF, W);
+      push_tile<TX, TY, TZ>(P1, local, s0, s1, sF, W);
     }
     // every warp is done with this field stage (and the staged parameters)
     // before they are refilled
-    if (__syncthreads_or(W.dead)) {
-      // a record chunk never arrived: report, wait (bounded) for this warp's
-      // copies still in flight and for the prefetched field stage, give up
-      if (tid == 0) atomicOr(err0, ERRBIT_TIMEOUT);
-      for (int b = 0; b < 2; ++b)
-        if (W.inflight & (1u << b)) mbar_wait_bounded(W.cbar + b, (W.phase >> b) & 1u);
-      if (tile + (int)gridDim.x < ntiles)
-        mbar_wait_bounded(bar + (stage ^ 1), ((it + 1) >> 1) & 1);
-      return;
-    }
+    __syncthreads();
   }
   if constexpr (MULTI) {
     for (int job = 0; job < J.njobs; ++job) {
@@ -1336,19 +1267,18 @@ __device__ __forceinline__ int tile_of_order(const CycleParams &P, int o) {
 }
 
 // Shared memory of the fused cycle: the push's field stages, then its record
-// staging and ring or the deposit's per-cell sums (whichever is larger; the
-// two are used at different times), then the barriers.
-template <int TX, int TY, int TZ, int MINB>
+// staging or the deposit's per-cell sums (whichever is larger; the two are
+// used at different times), then the barriers.
+template <int TX, int TY, int TZ>
 __host__ __device__ constexpr size_t fused_rec_bytes() {
-  return (size_t)(SIM_NW * 64 + SIM_NW * 2 * ring_half<MINB>() * 2) * 16 >
-                 (size_t)Tile<TX, TY, TZ>::TC * 80 * 4
-             ? (size_t)(SIM_NW * 64 + SIM_NW * 2 * ring_half<MINB>() * 2) * 16
+  return (size_t)SIM_NW * 64 * 16 > (size_t)Tile<TX, TY, TZ>::TC * 80 * 4
+             ? (size_t)SIM_NW * 64 * 16
              : (size_t)Tile<TX, TY, TZ>::TC * 80 * 4;
 }
-template <int TX, int TY, int TZ, int MINB>
+template <int TX, int TY, int TZ>
 __host__ __device__ constexpr size_t fused_smem() {
-  return 2 * (size_t)Tile<TX, TY, TZ>::SF * 4 + fused_rec_bytes<TX, TY, TZ, MINB>() +
-         (2 + 2 * SIM_NW) * sizeof(uint64_t);
+  return 2 * (size_t)Tile<TX, TY, TZ>::SF * 4 + fused_rec_bytes<TX, TY, TZ>() +
+         2 * sizeof(uint64_t);
 }
 
 // Thread 0 waits (bounded) until every neighbour of `tile` (itself included,
@@ -1388,7 +1318,7 @@ __device__ __forceinline__ bool wait_neighbours(const CycleParams &P, const int 
 // The fused cycle (the batching form's one launch per cycle), all species.
 // Persistent CTAs, all resident (cooperative launch), take the tiles in the
 // launch order above: at step k a CTA pushes its k-th tile (as k_push does:
-// TMA-staged fields, record ring, particles written into their new cells'
+// TMA-staged fields, particles written into their new cells'
 // buckets) and publishes it, then deposits its tile from lag steps earlier
 // (as k_deposit does, with coherent loads) once the 27 tiles around it are
 // published, whose pushes are the only ones that write into its buckets. The
@@ -1406,24 +1336,20 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
     k_cycle(const __grid_constant__ CUtensorMap fmap, const __grid_constant__ CycleParams P,
             const __grid_constant__ FusedAux X) {
   using T = Tile<TX, TY, TZ>;
-  constexpr int RH = ring_half<MINB>();
   static_assert(T::TC % SIM_NW == 0 && T::TC / SIM_NW <= 32,
                 "cells per warp must fit a warp's lanes");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float *sF0 = reinterpret_cast<float *>(smem_raw);                 // 2 stages x SF
   float4 *sRec = reinterpret_cast<float4 *>(sF0 + 2 * T::SF);       // NW x 64 staged records
-  float4 *sBuf = sRec + SIM_NW * 64;                                // NW x 2 x RH records
   uint64_t *bar = reinterpret_cast<uint64_t *>(reinterpret_cast<unsigned char *>(sRec) +
-                                               fused_rec_bytes<TX, TY, TZ, MINB>());   // 2 + 2 NW
-  // the deposit's per-cell sums reuse the record staging and ring (idle
+                                               fused_rec_bytes<TX, TY, TZ>());   // 2
+  // the deposit's per-cell sums reuse the record staging (idle
   // between two tiles' pushes; the field stages stay untouched)
   float2 *sCell = reinterpret_cast<float2 *>(sRec);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5;
   PushWarp W;
   W.wrec = sRec + warp * 64;
-  W.ring = sBuf + warp * 2 * RH * 2;
-  W.cbar = bar + 2 + warp * 2;
   if (smem_addr(sF0) & 127u) {
     if (tid == 0) atomicOr(P.err, ERRBIT_SMEM_ALIGN);
     return;
@@ -1431,10 +1357,6 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
   if (tid == 0) {
     mbar_init(bar, 1);
     mbar_init(bar + 1, 1);
-  }
-  if (lane == 0) {
-    mbar_init(W.cbar, 1);
-    mbar_init(W.cbar + 1, 1);
   }
   __syncthreads();
 
@@ -1446,6 +1368,7 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
     fence_proxy_async();
     mbar_expect_tx(bar + stage, box_bytes);
     tma_load_4d(sF0 + stage * T::SF, &fmap, 0, z * TZ, y * TY, x * TX, bar + stage);
+    tma_load_4d(sF0 + stage * T::SF + T::SH, &fmap, 4, z * TZ, y * TY, x * TX, bar + stage);
   };
   const int first = blockIdx.x;
   if (tid == 0 && first < ntiles) issue(tile_of_order(P, first), 0);
@@ -1465,14 +1388,7 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
         return;
       }
       const int tile = tile_of_order(P, o);
-      push_tile<TX, TY, TZ, RH, true>(P, tile, 0, P.ns, sF0 + stage * T::SF, W);
-      if (__syncthreads_or(W.dead)) {
-        if (tid == 0) atomicOr(P.err, ERRBIT_TIMEOUT);
-        for (int b = 0; b < 2; ++b)
-          if (W.inflight & (1u << b)) mbar_wait_bounded(W.cbar + b, (W.phase >> b) & 1u);
-        if (o + G < ntiles) mbar_wait_bounded(bar + (stage ^ 1), ((it + 1) >> 1) & 1);
-        return;
-      }
+      push_tile<TX, TY, TZ, true>(P, tile, 0, P.ns, sF0 + stage * T::SF, W);
       // publish: every thread's stores, then the flag
       __threadfence();
       __syncthreads();
@@ -1651,7 +1567,8 @@ __global__ void k_fill(GridScalars g, int nty, int ntz, const float *__restrict_
     to_cell(z[i], g.invdz, g.nzc, cz, oz, bad);
     const int key = tile_key<TX, TY, TZ>(cx, cy, cz, nty, ntz);
     const int slot = atomicAdd(S.cout + key, 1);
-    lost |= put_at(S, key, S.base[key], S.base[key + 1], slot, make_float4(ox, oy, oz, q[i]),
+    const long long d0 = S.base[key];
+    lost |= put_at(S, key, d0, (int)(S.base[key + 1] - d0), slot, make_float4(ox, oy, oz, q[i]),
                    make_float4(u[i], v[i], w[i], 0.f));
   }
   if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
@@ -1678,16 +1595,18 @@ __global__ void k_relayout(const long long *__restrict__ obase, const float4 *__
     int first = 0;
     if (lane == 0) first = atomicAdd(S.cout + key, c);
     first = __shfl_sync(FULL, first, 0);
-    const long long nb = S.base[key], ne = S.base[key + 1];
+    const long long nb = S.base[key];
+    const int cap = (int)(S.base[key + 1] - nb);
     for (int j = lane; j < c; j += 32)
-      lost |= put_at(S, (int)key, nb, ne, first + j, rin[2 * (ob + j)], rin[2 * (ob + j) + 1]);
+      lost |= put_at(S, (int)key, nb, cap, first + j, rin[2 * (ob + j)], rin[2 * (ob + j) + 1]);
   }
   const int on = min(*ocin, ocap_in);
   for (long j = blockIdx.x * (long)blockDim.x + threadIdx.x; j < on;
        j += (long)gridDim.x * blockDim.x) {
     const int key = okin[j];
     const int slot = atomicAdd(S.cout + key, 1);
-    lost |= put_at(S, key, S.base[key], S.base[key + 1], slot, oin[2 * j], oin[2 * j + 1]);
+    const long long nb = S.base[key];
+    lost |= put_at(S, key, nb, (int)(S.base[key + 1] - nb), slot, oin[2 * j], oin[2 * j + 1]);
   }
   if (lost) atomicOr(err, ERRBIT_LOST);
 }
@@ -1905,10 +1824,10 @@ int encode_field_map(spb_sim *s) {
       return fail(SPB_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
     encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
   }
-  // dims innermost first: 8 channels, z nodes, y nodes, x nodes
+  // dims innermost first: 8 channels (copied four at a time), z, y, x nodes
   const cuuint64_t dims[4] = {8, (cuuint64_t)s->nzn, (cuuint64_t)s->nyn, (cuuint64_t)s->nxn};
   const cuuint64_t strides[3] = {32, 32ull * s->nzn, 32ull * s->nzn * s->nyn};
-  const cuuint32_t box[4] = {8, (cuuint32_t)(s->tile[2] + 3), (cuuint32_t)(s->tile[1] + 3),
+  const cuuint32_t box[4] = {4, (cuuint32_t)(s->tile[2] + 3), (cuuint32_t)(s->tile[1] + 3),
                              (cuuint32_t)(s->tile[0] + 3)};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = encode(&s->fmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, s->fields8, dims, strides,
@@ -1923,9 +1842,7 @@ int encode_field_map(spb_sim *s) {
 template <int TX, int TY, int TZ, int MINB>
 size_t push_smem(bool multi = false) {
   return 2 * (size_t)Tile<TX, TY, TZ>::SF * 4 + (size_t)SIM_NW * 64 * sizeof(float4) +
-         (size_t)SIM_NW * 2 * ring_half<MINB>() * 2 * sizeof(float4) +
-         (multi ? sizeof(CycleParams) : 0) +
-         (2 + 2 * SIM_NW) * sizeof(uint64_t);
+         (multi ? sizeof(CycleParams) : 0) + 2 * sizeof(uint64_t);
 }
 template <int TX, int TY, int TZ>
 size_t deposit_smem(bool multi = false, bool exact = false) {
@@ -2082,7 +1999,7 @@ int launch_cycle_fused(spb_sim *s, cudaStream_t st) {
   }
   const int ntiles = s->nt[0] * s->nt[1] * s->nt[2];
   SPB_CUDA(cudaMemsetAsync(s->fused_done, 0, (ntiles + 2) * sizeof(int), st));
-  const size_t sm = fused_smem<TX, TY, TZ, MINB>();
+  const size_t sm = fused_smem<TX, TY, TZ>();
   static int occ = -1;
   if (occ < 0) {
     SPB_CUDA(cudaFuncSetAttribute(k_cycle<TX, TY, TZ, MINB>,
