@@ -74,6 +74,7 @@ struct spb_sim {
   bool fields_set = false;
   cudaEvent_t created = nullptr;  // the zeroing queued at creation is done
   int cycles_since_check = 0;
+  int *h_ovf = nullptr;           // pinned: the species' overflow counters at a check
   // CUDA graphs of one cycle's launches, keyed by the species' buffer parities;
   // captured and replayed on gstream, ordered after the caller's stream
   std::map<unsigned, cudaGraphExec_t> graphs;
