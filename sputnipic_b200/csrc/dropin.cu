@@ -604,6 +604,7 @@ extern "C" int spb_particle_sort(struct parameters *param, struct particles *par
     const long nb = 1 + ((nc[a] - 1) / param->sort_cps);
     B.nb[a] = (int)nb;
     B.dist[a] = (float)(L[a] / (double)(float)nb);   // FPpart dist = Lx / (FPpart)n_bin
+    B.inv[a] = (float)(1.0 / (double)B.dist[a]);
   }
   Species *sp = nullptr;
   if (int rc = get_species(part, &sp)) return rc;

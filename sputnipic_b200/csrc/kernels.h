@@ -15,6 +15,7 @@ int launch_plain_mover(const GeomDev &g, const PushDev &p, const PackedFields &F
 struct SortBins {
   int nb[3];       // bins per axis
   float dist[3];   // bin widths, rounded to float as the reference does
+  float inv[3];    // 1 / dist
 };
 size_t particle_sort_scratch_bytes(long n);
 // Sorts arr[0..6] (x, y, z, u, v, w, q; n each) by bin, stably; tmp: seven

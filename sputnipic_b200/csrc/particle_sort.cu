@@ -27,20 +27,30 @@ constexpr int RS_WARPS = RS_TPB / 32;
 constexpr int RS_CHUNK = RS_TPB * 16;        // elements per CTA and pass
 constexpr unsigned FULLM = 0xffffffffu;
 
+// floorf(x / dist) as the reference rounds it (the quotient to float first), from
+// the product with 1 / dist, which is within two units in the last place of the
+// quotient: unless it lies within four of an integer, both have the same floor.
+// The pass over 2.4M particles: 23 -> 18 us.
+__device__ __forceinline__ float bin_of(float x, float dist, float inv) {
+  const float q = __fmul_rn(x, inv);
+  if (!(fabsf(q - rintf(q)) > fabsf(q) * 4.8e-7f)) return floorf(__fdiv_rn(x, dist));
+  return floorf(q);
+}
+
 __global__ void k_bin_keys(const float *__restrict__ x, const float *__restrict__ y,
                            const float *__restrict__ z, long n, SortBins B,
                            unsigned *__restrict__ key, unsigned *__restrict__ idx) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
        i += (long)gridDim.x * blockDim.x) {
-    const float fx = floorf(__fdiv_rn(x[i], B.dist[0]));
-    const float fy = floorf(__fdiv_rn(y[i], B.dist[1]));
-    const float fz = floorf(__fdiv_rn(z[i], B.dist[2]));
+    const float fx = bin_of(x[i], B.dist[0], B.inv[0]);
+    const float fy = bin_of(y[i], B.dist[1], B.inv[1]);
+    const float fz = bin_of(z[i], B.dist[2], B.inv[2]);
     // out of the bin zone (or not a number): the last bin
     const bool in = fx >= 0.0f && fx < (float)B.nb[0] && fy >= 0.0f && fy < (float)B.nb[1] &&
                     fz >= 0.0f && fz < (float)B.nb[2];
-    const long k = in ? (long)fz + (long)fy * B.nb[2] + (long)fx * B.nb[2] * B.nb[1]
-                      : (long)B.nb[0] * B.nb[1] * B.nb[2];
-    key[i] = (unsigned)k;
+    // fewer than 2^32 bins (device_particle_sort)
+    const unsigned n2 = (unsigned)B.nb[2], n12 = (unsigned)B.nb[1] * n2;
+    key[i] = in ? (unsigned)fz + (unsigned)fy * n2 + (unsigned)fx * n12 : (unsigned)B.nb[0] * n12;
     idx[i] = (unsigned)i;
   }
 }

@@ -65,3 +65,24 @@ def test_final_velocity_and_reciprocal():
     slow = (low >= 0x0FFFFFFE) & (low <= 0x10000002)
     assert np.abs(q.view(np.int64) - (1.0 / d).view(np.int64)).max() <= 1
     assert np.array_equal(q[~slow].astype(np.float32), (1.0 / d)[~slow].astype(np.float32))
+
+
+@pytest.mark.parametrize("nb,L", [(33, 20.0), (1, 7.7), (64, 1e-3), (1000, 3.3), (65536, 1e3)])
+def test_sort_bins_from_products(nb, L):
+    """floor(x / dist) in float arithmetic against floor(x * (1 / dist)) where the latter is used:
+    farther than 4.8e-7 of its value from an integer."""
+    rng = np.random.default_rng(nb)
+    dist = np.float32(L / np.float32(nb))
+    inv = np.float32(1.0 / np.float64(dist))
+    x = (rng.integers(-2, nb + 3, 200000) * np.float64(dist)).astype(np.float32)
+    for _ in range(6):
+        k = rng.integers(-1, 2, x.size)
+        x = np.where(k < 0, np.nextafter(x, np.float32(-1e9)),
+                     np.where(k > 0, np.nextafter(x, np.float32(1e9)), x))
+    x = np.concatenate([x, (rng.uniform(-1, 1.1, 200000) * L).astype(np.float32),
+                        np.float32([0.0, -0.0, 1e-45, -1e-45, 1e30, -1e30])])
+    ref = np.floor(x / dist)
+    q = x * inv
+    used = np.abs(q - np.rint(q)) > np.abs(q) * np.float32(4.8e-7)
+    assert used.mean() > 0.3
+    assert np.array_equal(np.floor(q[used]), ref[used])
