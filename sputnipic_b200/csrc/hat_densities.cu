@@ -27,6 +27,7 @@
 #include "../../include/sputnipic_ref_layout.h"
 #include "common.h"
 #include "grid_ctx.h"
+#include "kernels.h"
 
 namespace spb {
 namespace {
@@ -133,9 +134,10 @@ __device__ __forceinline__ double d4_planes(const HatGeom &g, const Plane6<T> &l
 // a cell costs 24 loads (four nodes of six components) instead of the 72 that
 // its nine stencils read one by one: those kept the L1 pipe busy (an unaligned
 // row of 32 doubles takes three passes). 128x64x64 cells, 4 species, FP64: 62 ->
-// 46 us; with the guard fills gone the whole call 168 -> 110 us.
+// 46 us; with the guard fills gone the whole call 168 -> 110 us. Register caps
+// for four (double) and five (float) CTAs per SM: float 83 -> 74 us.
 template <typename T>
-__global__ void __launch_bounds__(128) k_hat_div_tensor(HatGeom g, const __grid_constant__ Species6<T> S, T alfa, int run) {
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 5) k_hat_div_tensor(HatGeom g, const __grid_constant__ Species6<T> S, T alfa, int run) {
   const int is = blockIdx.y;
   const int my = g.nyc - 2, mz = g.nzc - 2;
   const unsigned columns = (unsigned)(((long)my * mz + 127) / 128);   // CTAs per run
@@ -294,8 +296,8 @@ int hat_densities(const spb_hat_desc *d, const T *const *mom, const T *const B[3
   const long cells = (long)g.nxc * g.nyc * g.nzc, nodes = (long)g.nxn * g.nyn * g.nzn;
   const int ns = d->ns;
   // three centre temporaries per species (their guard cells are never written)
-  T *tc = nullptr;
-  SPB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&tc), 3 * ns * cells * sizeof(T), st));
+  T *const tc = static_cast<T *>(pool_alloc(3 * ns * cells * sizeof(T), st));
+  if (!tc) return fail(SPB_ERR_CUDA, "spb_hat_densities: scratch allocation failed");
   Species6<T> S;   // kernel parameters (copied at launch)
   std::memset(&S, 0, sizeof(S));
   for (int is = 0; is < ns; ++is) {
@@ -322,7 +324,7 @@ int hat_densities(const spb_hat_desc *d, const T *const *mom, const T *const B[3
                                                        d->dt * d->th, rhoh);
   if (cudaGetLastError() != cudaSuccess) rc = fail(SPB_ERR_CUDA, "spb_hat_densities: launch");
   g_launches += 3;
-  cudaFreeAsync(tc, st);
+  pool_free(tc, st);
   return rc;
 }
 
@@ -369,8 +371,7 @@ int hat_dropin(struct interpDens_aux *aux, struct interpDensNet *idn,
   T *buf = nullptr;
   const size_t bytes = ((size_t)(nin + 3) * nodes + 2 * (size_t)cells) * sizeof(T);
   int rc = SPB_OK;
-  if (cudaMallocAsync(reinterpret_cast<void **>(&buf), bytes, st) != cudaSuccess) {
-    cudaGetLastError();
+  if (!(buf = static_cast<T *>(pool_alloc(bytes, st)))) {
     cudaStreamDestroy(st);
     return fail(SPB_ERR_ALLOC, "calculateHatDensities: device allocation failed");
   }
@@ -409,7 +410,7 @@ int hat_dropin(struct interpDens_aux *aux, struct interpDensNet *idn,
     if (cudaMemcpyAsync(dst[a], srcd[a], cnt[a] * sizeof(T), cudaMemcpyDeviceToHost, st) !=
         cudaSuccess)
       rc = fail(SPB_ERR_CUDA, "calculateHatDensities: download");
-  cudaFreeAsync(buf, st);
+  pool_free(buf, st);
   if (cudaStreamSynchronize(st) != cudaSuccess && rc == SPB_OK)
     rc = fail(SPB_ERR_CUDA, "calculateHatDensities: stream");
   cudaStreamDestroy(st);
