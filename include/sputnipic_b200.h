@@ -72,12 +72,16 @@ const char *spb_version(void);
 long spb_launch_count(void);
 
 /* How the plain interpP2G / mover_interp deposits (process-wide):
+ * it concerns deposits of fewer than 65,536 particles and those that cannot
+ * get the scratch of the sorted deposit (32 bytes per particle of a chunk of
+ * at most 2^26 particles, halved until it can be had, from the device's
+ * stream-ordered pool), which adds straight into the ten arrays.
  * SPB_DEPOSIT_ACCUMULATOR (default) adds into a node-interleaved buffer of
- * 48 bytes per node from the device's stream-ordered pool, then into the
- * ten moment arrays (fewer L2 transactions); SPB_DEPOSIT_DIRECT adds straight
- * into the ten arrays and needs no memory. The accumulator form falls back to
- * the direct one when its buffer cannot be allocated. Returns the previous
- * mode, or SPB_ERR_INVALID for an unknown mode. */
+ * 48 bytes per node from the pool, then into the ten moment arrays (fewer L2
+ * transactions); SPB_DEPOSIT_DIRECT adds straight into the ten arrays. The
+ * accumulator form falls back to the direct one when its buffer cannot be
+ * allocated. Returns the previous mode, or SPB_ERR_INVALID for an unknown
+ * mode. */
 enum { SPB_DEPOSIT_ACCUMULATOR = 0, SPB_DEPOSIT_DIRECT = 1 };
 int spb_set_plain_deposit_mode(int mode);
 
@@ -222,14 +226,13 @@ int spb_grid_mover(spb_grid_ctx *ctx, const spb_push *push, float *x, float *y,
                    float *z, float *u, float *v, float *w, long n, void *stream);
 /* interpP2G over n particles: ADDS into mom[0..9] (device, nodes floats each,
  * anywhere in memory; order rhon, Jx, Jy, Jz, pxx, pxy, pxz, pyy, pyz, pzz).
- * The deposit accumulates into a node-interleaved buffer (48 bytes per node,
- * from the device's stream-ordered pool on `stream`), which a second kernel
- * adds into the ten arrays. */
+ * From 65,536 particles on the deposit copies them into records grouped by
+ * cell (scratch from the device's stream-ordered pool on `stream`, see
+ * spb_set_plain_deposit_mode) and sums cell by cell. */
 int spb_grid_p2g(spb_grid_ctx *ctx, const float *x, const float *y,
                  const float *z, const float *u, const float *v, const float *w,
                  const float *q, long n, float *const mom[10], void *stream);
-/* mover_interp: move then deposit, one kernel (plus the accumulator fold, as
- * spb_grid_p2g). */
+/* mover_interp: spb_grid_mover, then spb_grid_p2g on the moved particles. */
 int spb_grid_mover_interp(spb_grid_ctx *ctx, const spb_push *push, float *x,
                           float *y, float *z, float *u, float *v, float *w,
                           const float *q, long n, float *const mom[10],

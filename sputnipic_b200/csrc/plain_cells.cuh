@@ -38,7 +38,9 @@ __device__ __forceinline__ int clamp_cell(int i, int n, int &bad) {
 // exact, so a float product rounded down has the same floor (every integer
 // below 2^24 is a float, and rounding down cannot cross one), and compares
 // alike with the integers -1 and n - 2; cells outside the node array (and NaN)
-// take the general path, which flags them.
+// take the general path, which flags them. The floor itself is an add rounded
+// down against 1.5 * 2^23, whose neighbouring floats are the integers (no axis
+// has 2^22 nodes): a conversion per axis kept the conversion unit half busy.
 template <bool FLOAT_CELLS>
 __device__ __forceinline__ void deposit_cell(const GeomDev &g, float x, float y, float z, int &ix,
                                              int &iy, int &iz, int &bad) {
@@ -46,9 +48,10 @@ __device__ __forceinline__ void deposit_cell(const GeomDev &g, float x, float y,
     const float px = __fmul_rd(x, g.invdx), py = __fmul_rd(y, g.invdy),
                 pz = __fmul_rd(z, g.invdz);
     if (px >= -1.0f && px < g.nxf && py >= -1.0f && py < g.nyf && pz >= -1.0f && pz < g.nzf) {
-      ix = 2 + __float2int_rd(px);
-      iy = 2 + __float2int_rd(py);
-      iz = 2 + __float2int_rd(pz);
+      constexpr float M = 12582912.0f;   // 1.5 * 2^23
+      ix = 2 + __float_as_int(__fadd_rd(px, M)) - __float_as_int(M);
+      iy = 2 + __float_as_int(__fadd_rd(py, M)) - __float_as_int(M);
+      iz = 2 + __float_as_int(__fadd_rd(pz, M)) - __float_as_int(M);
       return;
     }
   }

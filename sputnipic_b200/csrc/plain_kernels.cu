@@ -12,10 +12,9 @@
 // bit-identical to the reference CPU code; moments differ only by the order
 // of the FP32 additions.
 //
-// Launch shape. One thread per particle, 256 threads per block: the particle
-// SoA streams through once (coalesced 4-byte loads per array per warp), the
-// 8-node gathers hit the packed fields, which stay L2-resident (14 MB at
-// 128x64x64 cells).
+// Launch shape. One thread per particle: the particle SoA streams through once
+// (coalesced 4-byte loads per array per warp), the 8-node gathers hit the packed
+// fields, which stay L2-resident (28 MB at 128x64x64 cells).
 #include "bc_fold.cuh"
 #include "grid_ctx.h"
 #include "kernels.h"

@@ -14,8 +14,8 @@
 // deposit 4-byte gathers through it, 4.5 L2 sectors per particle in arrays
 // near cell order and up to 7 in others, and a warp reduction per run of a
 // cell's particles. 65.5M particles in cell order, 125 per cell, zeroing and
-// applyBCids included: 2352 -> 1586 us (count 180, copy 706, sum 650); two
-// species of 2.4M some cycles after the last sort, 27 per cell: 432 -> 237 us.
+// applyBCids included: 2352 -> 1455 us (count 150, copy 680, sum 600); two
+// species of 2.4M some cycles after the last sort, 27 per cell: 432 -> 232 us.
 //
 // Cells are numbered tile by tile (8 x 4 x 4 cells; a CTA of the last launch
 // takes a tile), over the nxn - 1 cells per axis that node pairs (i - 1, i)
@@ -134,15 +134,11 @@ __global__ void __launch_bounds__(TPB) k_p2g_records(GeomDev g, int nty, int ntz
   const int lane = threadIdx.x & 31;
   int bad = 0;
   for (long base = (long)blockIdx.x * TPB; base < n; base += (long)gridDim.x * TPB) {
-    const long i = base + threadIdx.x;
-    const bool valid = i < n;
-    int key = -1;
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-    if (valid) {
-      a = make_float4(P.p[0][i], P.p[1][i], P.p[2][i], P.p[6][i]);
-      b = make_float4(P.p[3][i], P.p[4][i], P.p[5][i], 0.f);
-      key = cell_key<FLOAT_CELLS>(g, nty, ntz, a.x, a.y, a.z, bad);
-    }
+    const bool valid = base + threadIdx.x < n;
+    const long i = valid ? base + threadIdx.x : n - 1;   // every lane loads: no branch
+    const float4 a = make_float4(P.p[0][i], P.p[1][i], P.p[2][i], P.p[6][i]);
+    const float4 b = make_float4(P.p[3][i], P.p[4][i], P.p[5][i], 0.f);
+    const int key = valid ? cell_key<FLOAT_CELLS>(g, nty, ntz, a.x, a.y, a.z, bad) : -1;
     const unsigned peers = __match_any_sync(FULL, key);
     const int leader = __ffs(peers) - 1;
     unsigned at = 0;
@@ -204,11 +200,13 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
   };
 #pragma unroll 1
   for (int k = 0; k < trips; ++k) {
-    if (k && k % SUM_RUN == 0) put(k == SUM_RUN);
     // two records in flight while this one is summed; lanes past their count
     // add zero terms
     float4 na = a1, nb = b1;
     if (k + 2 < n1) ld_rec(rec + 2 * (k + 2), na, nb);
+    // (after the load is on its way: before it, the totals' round through
+    // shared memory kept the loads waiting, 55 us of 65.5M particles' 690)
+    if (k && k % SUM_RUN == 0) put(k == SUM_RUN);
     add_terms(acc, k < n1 ? a.w : 0.0f, X.y - a.x, a.x - X.x, Y.y - a.y, a.y - Y.x,
               (Z.y - a.z) * inv, (a.z - Z.x) * inv, b.x, b.y, b.z, 0);
     a = a1;
@@ -294,6 +292,7 @@ int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z,
   // on small grids the cells' records go to several CTAs: a thread walks its
   // cell's one after another, and with fewer tiles than CTAs fit (four per SM)
   // that walk is the launch's time; parts of at least eight records a cell
+  // (32x16x16 cells at 27 per cell: 22 -> 13 us)
   const long inner = std::max(1L, ceil_div(g.nxn - 3, TX)) *
                      std::max(1L, ceil_div(g.nyn - 3, TY)) *
                      std::max(1L, ceil_div(g.nzn - 3, TZ));
