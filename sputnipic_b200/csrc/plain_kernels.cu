@@ -468,8 +468,8 @@ __device__ __forceinline__ void deposit_lone(const GeomDev &g, const DepTarget &
 // warp_sum80 (one x half of the terms at a time), and one warp reduction and
 // 80 adds serve the whole group instead of one per 32 particles. Groups of up
 // to three particles deposit particle by particle (deposit_lone). A chunk
-// with more distinct cells than the table holds (unordered input) falls back
-// to the per-warp deposit of k_plain_p2g.
+// with more distinct cells than the table holds (unordered input) deposits
+// every particle by itself (deposit_lone).
 constexpr int GP_TPB = 256;
 constexpr int GP_PER_THREAD = 4;
 constexpr int GP_CHUNK = GP_TPB * GP_PER_THREAD;

@@ -41,11 +41,12 @@ DEPOSIT_MODES = {"accumulator": 0, "direct": 1}
 
 
 def set_plain_deposit_mode(mode: str) -> str:
-    """How the plain interpP2G / mover_interp deposits, process-wide
-    (spb_set_plain_deposit_mode): "accumulator" (a node-interleaved buffer
-    from the device pool, then added into the ten moment arrays; the default)
-    or "direct" (straight into the ten arrays, no extra memory). Returns the
-    previous mode."""
+    """How the plain interpP2G / mover_interp deposits where it does not sort
+    (fewer than 65,536 particles, or no scratch for the sorted deposit),
+    process-wide (spb_set_plain_deposit_mode): "accumulator" (a
+    node-interleaved buffer from the device pool, then added into the ten
+    moment arrays; the default) or "direct" (straight into the ten arrays).
+    Returns the previous mode."""
     if mode not in DEPOSIT_MODES:
         raise ValueError(f"unknown deposit mode {mode!r}")
     prev = _lib.load().spb_set_plain_deposit_mode(DEPOSIT_MODES[mode])
