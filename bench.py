@@ -656,10 +656,10 @@ def measure_hat(torch, wl, reps=10, warmup=3):
     peak = peaks()[0]
     achieved = algo / (ms * 1e-3) / 1e9
     return {"ms": ms, "species": ns, "dtype": "f64", "algorithmic_bytes": algo,
-            "achieved_gbs": achieved, "frac": achieved / peak, "launches": 9,
-            "note": "bit-identical to the reference's FP64 build; nine launches for all "
-                    "species (divergences, guard fills as gather + scatter, node pass, J hat "
-                    "guards, rho hat, rho hat guards)"}
+            "achieved_gbs": achieved, "frac": achieved / peak, "launches": 3,
+            "note": "bit-identical to the reference's FP64 build; three launches for all "
+                    "species (divergences, node pass, rho hat; guard nodes and cells with "
+                    "them)"}
 
 
 def run_e2e(args, wl, host_parts, host_f, world, dist):

@@ -155,8 +155,9 @@ __global__ void __launch_bounds__(TPB) k_p2g_records(GeomDev g, int nty, int ntz
 constexpr int SUM_RUN = 16;
 
 // One tile of cells (blockIdx.x) and one part of each cell's records
-// (blockIdx.y): thread t sums the records of cell t, the warp those above its quota (deposit_quota), and every node of the tile adds
-// its cells' sums into the moments. A term is f (q xi) eta (zeta invVOL),
+// (blockIdx.y): thread t sums the records of cell t, the warp those above its
+// quota (deposit_quota), and every node of the tile adds its cells' sums into
+// the moments. A term is f (q xi) eta (zeta invVOL),
 // summed in FP32; the second invVOL multiplies a node's sum once (the reference
 // multiplies every term by both): fewer roundings than its own. (q invVOL
 // would round alike for all particles of equal charge: a bias, not noise.)
