@@ -153,7 +153,9 @@ int spb_particle_sort(struct parameters *param, struct particles *part, struct g
  * on device arrays: mom holds ns*10 device pointers (species-major, the
  * interpP2G moment order; entries 1..9 are read), B the three magnetic
  * field node arrays, rhoc the centre array [nxc][nyc][nzc] (guards
- * included); outputs as the drop-in's. Asynchronous on `stream`. */
+ * included); outputs as the drop-in's. An output may be an input array: J hat
+ * any of the moments or B, rho hat rhoc, a moment or B. Asynchronous on
+ * `stream`. */
 struct interpDens_aux;
 #define SPB_HAT_MAX_SPECIES 16
 typedef struct spb_hat_desc {

@@ -14,6 +14,11 @@
 // J hat) each take the value of one inner cell (guard_source), so they are
 // read, or computed, where that cell is: no fill passes.
 //
+// In place. J hat may be written over J or B, and rho hat over rho_c. A guard
+// entry's thread would then read an inner entry that its own thread may already
+// have overwritten, so such a call computes the inner entries only, each from
+// its own, and copies the guards afterwards (k_hat_guards).
+//
 // Arithmetic. This file is compiled with -fmad=false and follows the C
 // promotions of the reference expressions: the stencils' .25 * (a - b) * inv
 // terms and the .125 interpolation scale are double, rounded to the array
@@ -200,10 +205,11 @@ struct Out3 {
 // rotated by the species' beta B and added into J hat, which starts at 0 (the
 // reference's per-species accumulation, in registers). A guard node computes
 // the node that its value comes from, and guard cells are read where theirs
-// does. Four CTAs per SM (at most 64 registers), for the same reason.
+// does; without `guards` a guard node is left alone. Four CTAs per SM (at most
+// 64 registers), for the same reason.
 template <typename T>
 __global__ void __launch_bounds__(256, 4) k_hat_pidot(HatGeom g, const __grid_constant__ Species6<T> S, int ns, Vec3<T> B,
-                            Out3<T> JH) {
+                            Out3<T> JH, bool guards) {
   const long nodes = (long)g.nxn * g.nyn * g.nzn;
   for (long n = blockIdx.x * (long)blockDim.x + threadIdx.x; n < nodes;
        n += (long)gridDim.x * blockDim.x) {
@@ -211,6 +217,7 @@ __global__ void __launch_bounds__(256, 4) k_hat_pidot(HatGeom g, const __grid_co
     const int j = guard_source((int)((n / g.nzn) % g.nyn), g.nyn, 2, g.per[1]);
     const int k = guard_source((int)(n % g.nzn), g.nzn, 2, g.per[2]);
     const long m = nidx(g, i, j, k);
+    if (!guards && m != n) continue;
     // the node's upper cell, and the steps to its lower ones per axis
     const int i0 = guard_source(i, g.nxc, 1, g.per[0]), j0 = guard_source(j, g.nyc, 1, g.per[1]),
               k0 = guard_source(k, g.nzc, 1, g.per[2]);
@@ -251,22 +258,47 @@ __global__ void __launch_bounds__(256, 4) k_hat_pidot(HatGeom g, const __grid_co
 }
 
 // rho hat = rho_c - dt theta div(J hat) on every cell; a guard cell computes
-// the cell that its value comes from.
+// the cell that its value comes from, or nothing without `guards`.
 template <typename T>
-__global__ void k_hat_rho(HatGeom g, Vec3<T> JH, const T *__restrict__ rhoc, double dt_th,
-                          T *__restrict__ rhoh) {
+__global__ void k_hat_rho(HatGeom g, Vec3<T> JH, const T *rhoc, double dt_th, T *rhoh,
+                          bool guards) {
   const long cells = (long)g.nxc * g.nyc * g.nzc;
   for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < cells;
        c += (long)gridDim.x * blockDim.x) {
     const int i = guard_source((int)(c / ((long)g.nzc * g.nyc)), g.nxc, 1, g.per[0]);
     const int j = guard_source((int)((c / g.nzc) % g.nyc), g.nyc, 1, g.per[1]);
     const int k = guard_source((int)(c % g.nzc), g.nzc, 1, g.per[2]);
+    const long m = cidx(g, i, j, k);
+    if (!guards && m != c) continue;
     const T cx = (T)d4(g, JH.v[0], i, j, k, 0);
     const T cy = (T)d4(g, JH.v[1], i, j, k, 1);
     const T cz = (T)d4(g, JH.v[2], i, j, k, 2);
     const T dv = cx + cy + cz;
-    rhoh[c] = (T)((double)rhoc[cidx(g, i, j, k)] - dt_th * (double)dv);
+    rhoh[c] = (T)((double)rhoc[m] - dt_th * (double)dv);
   }
+}
+
+// The guard entries of n0 x n1 x n2 arrays, each from the inner entry
+// that its value comes from (blockIdx.y: the array).
+template <typename T>
+__global__ void k_hat_guards(int n0, int n1, int n2, int s, HatGeom g, Out3<T> A) {
+  T *const a = A.v[blockIdx.y];
+  const long n = (long)n0 * n1 * n2;
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n;
+       t += (long)gridDim.x * blockDim.x) {
+    const long i = guard_source((int)(t / ((long)n2 * n1)), n0, s, g.per[0]);
+    const int j = guard_source((int)((t / n2) % n1), n1, s, g.per[1]);
+    const int k = guard_source((int)(t % n2), n2, s, g.per[2]);
+    const long m = (i * n1 + j) * n2 + k;
+    if (m != t) a[t] = a[m];
+  }
+}
+
+// Whether the na entries at a and the nb at b share memory.
+template <typename T>
+bool share(const T *a, long na, const T *b, long nb) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + nb * sizeof(T) && y < x + na * sizeof(T);
 }
 
 int blocks_for(long n, int tpb) {
@@ -318,12 +350,26 @@ int hat_densities(const spb_hat_desc *d, const T *const *mom, const T *const B[3
   const dim3 grid((unsigned)(ceil_div((long)(g.nyc - 2) * (g.nzc - 2), 128) *
                              ceil_div(g.nxc - 2, run)), (unsigned)ns);
   k_hat_div_tensor<T><<<grid, 128, 0, st>>>(g, S, alfa, run);
+  const Out3<T> JH{{jxh, jyh, jzh}};
+  bool j_over = false;   // J hat over the inputs of its own pass
+  for (int r = 0; r < 3; ++r) {
+    for (int c = 0; c < 3; ++c) j_over |= share(JH.v[r], nodes, B[c], nodes);
+    for (int is = 0; is < ns; ++is)
+      for (int c = 0; c < 3; ++c) j_over |= share(JH.v[r], nodes, S.j[is][c], nodes);
+  }
+  const bool rho_over = share(rhoh, cells, rhoc, cells);
   k_hat_pidot<T><<<blocks_for(nodes, 256), 256, 0, st>>>(g, S, ns, Vec3<T>{{B[0], B[1], B[2]}},
-                                                         Out3<T>{{jxh, jyh, jzh}});
+                                                         JH, !j_over);
+  if (j_over)
+    k_hat_guards<T><<<dim3(blocks_for(nodes, 256), 3), 256, 0, st>>>(g.nxn, g.nyn, g.nzn, 2, g,
+                                                                     JH);
   k_hat_rho<T><<<blocks_for(cells, 256), 256, 0, st>>>(g, Vec3<T>{{jxh, jyh, jzh}}, rhoc,
-                                                       d->dt * d->th, rhoh);
+                                                       d->dt * d->th, rhoh, !rho_over);
+  if (rho_over)
+    k_hat_guards<T><<<blocks_for(cells, 256), 256, 0, st>>>(g.nxc, g.nyc, g.nzc, 1, g,
+                                                            Out3<T>{{rhoh, nullptr, nullptr}});
   if (cudaGetLastError() != cudaSuccess) rc = fail(SPB_ERR_CUDA, "spb_hat_densities: launch");
-  g_launches += 3;
+  g_launches += 3 + j_over + rho_over;
   pool_free(tc, st);
   return rc;
 }

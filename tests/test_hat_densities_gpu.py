@@ -92,3 +92,39 @@ def test_gem_grid_fp64_equals_oracle(cuda):
     got = run_device(cuda, wl, qom, 1.0, 64, mom, fields, rhoc)
     for g, r in zip(got, ref):
         assert np.array_equal(g, r)
+
+
+@pytest.mark.parametrize("fp", [32, 64])
+@pytest.mark.parametrize("per", PERIODIC)
+@pytest.mark.parametrize("grid", [(8, 6, 5), (1, 1, 1), (40, 33, 21)])
+def test_outputs_over_inputs(cuda, fp, per, grid):
+    """J hat written over a species' J, over B or over pressures, and rho hat over rho_c or a
+    moment, give the bits that separate outputs get."""
+    import ctypes
+
+    from sputnipic_b200 import _lib
+    from sputnipic_b200.hat import hat_desc, hat_densities
+    torch = cuda
+    wl = W.small_gem(nxc=grid[0], nyc=grid[1], nzc=grid[2], periodic=tuple(bool(p) for p in per))
+    qom = [sp.qom for sp in wl.species[:3]]
+    dt = np.float32 if fp == 32 else np.float64
+    mom, fields, rhoc = W.hat_inputs(wl, seed=11, dtype=dt, ns=3)
+    T = lambda a: torch.from_numpy(np.ascontiguousarray(a).copy()).cuda()  # noqa: E731
+    desc = hat_desc(wl, 1.0, qom, fp)
+    want = hat_densities(desc, [[T(a) for a in sp] for sp in mom], [T(f) for f in fields[3:]],
+                         T(rhoc))
+    lib = _lib.load()
+    fn = lib.spb_hat_densities_f32 if fp == 32 else lib.spb_hat_densities_f64
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    for over in ("J0", "J2 turned", "B", "p1"):
+        m, B, rc = [[T(a) for a in sp] for sp in mom], [T(f) for f in fields[3:]], T(rhoc)
+        out = {"J0": m[0][1:4], "J2 turned": [m[2][3], m[2][1], m[2][2]], "B": list(B),
+               "p1": m[1][4:7]}[over]
+        rho = m[1][0] if over == "p1" else rc
+        mp = (ctypes.c_void_p * 30)(*[t.data_ptr() for sp in m for t in sp])
+        bp = (ctypes.c_void_p * 3)(*[t.data_ptr() for t in B])
+        _lib.check(fn(ctypes.byref(desc), mp, bp, ptr(rc), *[ptr(t) for t in out], ptr(rho),
+                      ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        torch.cuda.synchronize()
+        for got, w in zip([*out, rho], want):
+            assert torch.equal(got.view(-1)[:w.numel()], w), over
