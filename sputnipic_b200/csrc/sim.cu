@@ -2553,9 +2553,9 @@ extern "C" int spb_sim_create(const spb_sim_desc *d, spb_sim **out) {
     cudaGetLastError();
     return bail(fail(SPB_ERR_ALLOC, "spb_sim_create: device allocation failed"));
   }
-  // zeroed on the pool's stream; load_species, moments and check order
-  // themselves after it (spb_sim::created), since the caller's stream may be
-  // one that the default stream does not block
+  // zeroed on the pool's stream; whatever reads or writes that memory next
+  // comes after it (load_species on its stream, the others by wait_created),
+  // since the caller's stream may be one that the default stream does not block
   cudaStream_t pst = pool_stream();
   if (cudaMemsetAsync(s->d_err, 0, sizeof(int), pst) != cudaSuccess)
     return bail(fail(SPB_ERR_CUDA, "spb_sim_create: memset failed"));
@@ -2579,6 +2579,21 @@ extern "C" int spb_sim_create(const spb_sim_desc *d, spb_sim **out) {
 }
 
 namespace {
+// Waits on the host until the zeroing queued at creation is done: for calls
+// that may come before any species is loaded. On the host, because the moments'
+// address is handed out for use on any stream; relaxed, because the calling
+// thread may be capturing.
+cudaError_t wait_created(spb_sim *s) {
+  if (s->zeroed) return cudaSuccess;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return e;
+  e = cudaEventSynchronize(s->created);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  s->zeroed = e == cudaSuccess;
+  return e;
+}
+
 float elapsed(cudaEvent_t a, cudaEvent_t b) {
   float t = 0;
   if (cudaEventSynchronize(b) != cudaSuccess || cudaEventElapsedTime(&t, a, b) != cudaSuccess)
@@ -2929,7 +2944,7 @@ extern "C" int spb_sim_moments(spb_sim *s, int species, double *out, int on_devi
                                void *stream) {
   if (!s || !out || species < 0 || species >= (int)s->sp.size())
     return fail(SPB_ERR_INVALID, "spb_sim_moments: bad arguments");
-  if (!s->cycles_run) SPB_CUDA(cudaStreamWaitEvent((cudaStream_t)stream, s->created, 0));
+  SPB_CUDA(wait_created(s));
   SPB_CUDA(cudaMemcpyAsync(out, s->sp[species].mom, 10 * s->nodes * sizeof(double),
                            on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                            (cudaStream_t)stream));
@@ -2941,12 +2956,18 @@ extern "C" double *spb_sim_moments_device(spb_sim *s, int species) {
     fail(SPB_ERR_INVALID, "spb_sim_moments_device: bad arguments");
     return nullptr;
   }
+  const cudaError_t e = wait_created(s);
+  if (e != cudaSuccess) {
+    fail_cuda(e, "spb_sim_moments_device");
+    return nullptr;
+  }
   return s->sp[species].mom;
 }
 
 extern "C" int spb_sim_apply_bc_ids(spb_sim *s, int species, void *stream) {
   if (!s || species < 0 || species >= (int)s->sp.size())
     return fail(SPB_ERR_INVALID, "spb_sim_apply_bc_ids: bad arguments");
+  SPB_CUDA(wait_created(s));
   cudaStream_t st = (cudaStream_t)stream;
   const FoldGroups g = fold_groups(s->nxn, s->nyn, s->nzn, s->d.periodic);
   k_bc_fold64<<<dim3((unsigned)ceil_div(g.fx + g.fy + g.fz, 256), 10), 256, 0, st>>>(
@@ -3002,7 +3023,7 @@ int sim_status(int h) {
 
 extern "C" int spb_sim_check(spb_sim *s, void *stream) {
   if (!s) return fail(SPB_ERR_INVALID, "spb_sim_check: null simulation");
-  SPB_CUDA(cudaEventSynchronize(s->created));
+  SPB_CUDA(wait_created(s));
   SPB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
   int h = 0;
   SPB_CUDA(cudaMemcpy(&h, s->d_err, sizeof(int), cudaMemcpyDeviceToHost));

@@ -73,6 +73,7 @@ struct spb_sim {
   CUtensorMap fmap{};
   bool fields_set = false;
   cudaEvent_t created = nullptr;  // the zeroing queued at creation is done
+  bool zeroed = false;            // ... and the host has seen it
   int cycles_since_check = 0;
   int *h_ovf = nullptr;           // pinned: the species' overflow counters at a check
   // CUDA graphs of one cycle's launches, keyed by the species' buffer parities;

@@ -34,7 +34,6 @@ def test_bc_fold_bit_identical(cuda, grid):
         ref = m64.copy()
         oracle.CpuOracle("restated", 64).apply_bc_ids(setup, list(ref))
         sim = Simulation(wl, tile=(2, 2, 2), species=[0])
-        torch.cuda.synchronize()
         view = sim.moments_view(0)
         view.copy_(torch.from_numpy(m64))
         sim.apply_bc_ids(0)

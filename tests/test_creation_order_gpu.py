@@ -41,3 +41,40 @@ def test_zeroing_comes_before_the_callers_stream(cuda):
         assert float(a.norm()) > 0
         # the same particles' FP32 cell sums in any order (the bar of the precision form)
         assert float((a - b).norm() / a.norm()) <= 1e-5
+
+
+def test_moments_written_right_after_creation(cuda):
+    """A new simulation's moments may be written, folded and read at once, on the default stream
+    and on another one, also by a capturing stream: the zeroing comes first."""
+    torch = cuda
+    from sputnipic_b200.sim import Simulation
+
+    wl = W.small_gem(nxc=128, nyc=64, nzc=64, periodic=(False, False, False))   # 47 MB a species
+    ones = torch.ones(10, wl.nodes, dtype=torch.float64, device="cuda")
+    want = ones.view(10, wl.nxn, wl.nyn, wl.nzn).clone()
+    for axis in (1, 2, 3):
+        for at in (1, want.shape[axis] - 2):
+            plane = want.narrow(axis, at, 1)
+            inner = [slice(None)] + [slice(1, -1) if a != axis else slice(None) for a in (1, 2, 3)]
+            plane[tuple(inner)] *= 2
+    torch.cuda.synchronize()
+    for st in (torch.cuda.default_stream(), torch.cuda.Stream()):
+        for _ in range(3):
+            sim = Simulation(wl, species=[0, 1])
+            with torch.cuda.stream(st):
+                sim.moments_view(1).copy_(ones)
+                sim.apply_bc_ids(1, stream=st)
+                got = sim.moments(1, stream=st)
+            st.synchronize()
+            assert torch.equal(got.view_as(want), want)
+            assert sim.check(st) == 0
+            sim.close()
+    sim = Simulation(wl, species=[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        sim.apply_bc_ids(0, stream=torch.cuda.current_stream())
+    sim.moments_view(0).copy_(ones)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(sim.moments_view(0).view_as(want), want)
+    sim.close()
