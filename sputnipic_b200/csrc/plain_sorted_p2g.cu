@@ -201,15 +201,17 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
   };
 #pragma unroll 1
   for (int k = 0; k < trips; ++k) {
-    // two records in flight while this one is summed; lanes past their count
-    // add zero terms
+    // two records in flight while this one is summed
     float4 na = a1, nb = b1;
     if (k + 2 < n1) ld_rec(rec + 2 * (k + 2), na, nb);
     // (after the load is on its way: before it, the totals' round through
     // shared memory kept the loads waiting, 55 us of 65.5M particles' 690)
     if (k && k % SUM_RUN == 0) put(k == SUM_RUN);
-    add_terms(acc, k < n1 ? a.w : 0.0f, X.y - a.x, a.x - X.x, Y.y - a.y, a.y - Y.x,
-              (Z.y - a.z) * inv, (a.z - Z.x) * inv, b.x, b.y, b.z, 0);
+    // (lanes past their count add nothing: their last record with a charge of
+    // zero would turn an infinite product of its velocities into NaN)
+    if (k < n1)
+      add_terms(acc, a.w, X.y - a.x, a.x - X.x, Y.y - a.y, a.y - Y.x, (Z.y - a.z) * inv,
+                (a.z - Z.x) * inv, b.x, b.y, b.z, 0);
     a = a1;
     b = b1;
     a1 = na;

@@ -116,3 +116,30 @@ def test_more_than_one_chunk(cuda):
     # all terms positive: two FP32 sums of the same 2048 * 8 terms a node
     assert float(((whole - parts).norm(dim=1) / whole.norm(dim=1)).max()) < 2e-6
     ctx.close()
+
+
+@pytest.mark.parametrize("u", [3e19, float("inf"), float("-inf"), float("nan")])
+def test_infinite_products_stay_infinite(cuda, u):
+    """A velocity whose square overflows (or that is not finite) gives infinity and NaN in the
+    moments and at the nodes where the reference has them, whatever the counts of the other cells."""
+    torch = cuda
+    from sputnipic_b200 import device
+    rng = np.random.default_rng(5)
+    wl = W.GemWorkload(name="t", nxc=16, nyc=8, nzc=8, Lx=4.0, Ly=2.0, Lz=2.0)
+    p = particles(rng, wl, 66000, "anywhere")
+    # a cell of 24 such particles beside cells of about 64 others (in up to 8 parts)
+    p["x"][(p["x"] > 1.0) & (p["x"] < 1.25)] += np.float32(1.0)
+    for k, at in (("x", 1.1), ("y", 0.6), ("z", 0.9), ("u", u), ("v", 0.05), ("w", 0.1), ("q", 0.5)):
+        p[k][:24] = at
+    p["x"][:24] += np.arange(24, dtype=np.float32) / 256
+    ref = np.zeros((10, wl.nodes), np.float32)
+    oracle.CpuOracle("restated", 32).interp_p2g(oracle.setup_from(wl), p, list(ref))
+    ctx = device.GridContext(wl)
+    mom = torch.zeros(10, wl.nodes, device="cuda")
+    ctx.p2g(on_gpu(torch, p), mom)
+    assert ctx.check() == 0
+    got = mom.cpu().numpy()
+    ctx.close()
+    assert not np.isfinite(ref).all()
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    assert np.array_equal(np.where(np.isinf(got), got, 0), np.where(np.isinf(ref), ref, 0))
