@@ -149,9 +149,10 @@ __global__ void __launch_bounds__(TPB) k_p2g_records(GeomDev g, int nty, int ntz
   if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
 }
 
-// Particles that a lane sums before it adds them to the cell's totals: sums of
-// n terms one after another lose about n / 2 rounding errors' variance, sums
-// of runs of 16 of them 8 + n / 32, less than the warp's tree they replace.
+// Particles that a lane sums before they are added to the cell's totals (by the
+// warp, above the quota): sums of n terms one after another lose about n / 2
+// rounding errors' variance, sums of runs of 16 of them 8 + n / 32, less than
+// the warp's tree they replace.
 constexpr int SUM_RUN = 16;
 
 // One tile of cells (blockIdx.x) and one part of each cell's records
@@ -232,22 +233,26 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
       const float2 hX = make_float2(__shfl_sync(FULL, X.x, hl), __shfl_sync(FULL, X.y, hl));
       const float2 hY = make_float2(__shfl_sync(FULL, Y.x, hl), __shfl_sync(FULL, Y.y, hl));
       const float2 hZ = make_float2(__shfl_sync(FULL, Z.x, hl), __shfl_sync(FULL, Z.y, hl));
-#pragma unroll
-      for (int i = 0; i < 40; ++i) acc[i] = make_float2(0.f, 0.f);
-#pragma unroll 1
-      for (int o = Q; o < hc; o += 32) {
-        const int i = o + lane;
-        float4 ha = make_float4(0.f, 0.f, 0.f, 0.f), hb = ha;
-        if (i < hc) ld_rec(hrec + 2 * (long)i, ha, hb);
-        add_terms(acc, i < hc ? ha.w : 0.0f, hX.y - ha.x, ha.x - hX.x, hY.y - ha.y,
-                  ha.y - hY.x, (hZ.y - ha.z) * inv, (ha.z - hZ.x) * inv, hb.x, hb.y, hb.z, lane);
-      }
-      float r[5];
-      warp_sum80(acc, r, lane);
       float2 *dst = sCell + corner * 5 * TC + (tid & ~31) + hl;
+#pragma unroll 1
+      for (int o = Q; o < hc;) {
 #pragma unroll
-      for (int k = 0; k < 5; ++k)
-        if (k >= lo && k < hi) (half ? dst[k * TC].y : dst[k * TC].x) += r[k];
+        for (int i = 0; i < 40; ++i) acc[i] = make_float2(0.f, 0.f);
+        const int stop = min(o + 32 * SUM_RUN, hc);
+#pragma unroll 1
+        for (; o < stop; o += 32) {
+          const int i = o + lane;
+          float4 ha = make_float4(0.f, 0.f, 0.f, 0.f), hb = ha;
+          if (i < hc) ld_rec(hrec + 2 * (long)i, ha, hb);
+          add_terms(acc, i < hc ? ha.w : 0.0f, hX.y - ha.x, ha.x - hX.x, hY.y - ha.y,
+                    ha.y - hY.x, (hZ.y - ha.z) * inv, (ha.z - hZ.x) * inv, hb.x, hb.y, hb.z, lane);
+        }
+        float r[5];
+        warp_sum80(acc, r, lane);
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+          if (k >= lo && k < hi) (half ? dst[k * TC].y : dst[k * TC].x) += r[k];
+      }
     }
   }
   __syncthreads();

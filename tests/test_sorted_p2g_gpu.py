@@ -143,3 +143,27 @@ def test_infinite_products_stay_infinite(cuda, u):
     assert not np.isfinite(ref).all()
     assert np.array_equal(np.isnan(got), np.isnan(ref))
     assert np.array_equal(np.where(np.isinf(got), got, 0), np.where(np.isinf(ref), ref, 0))
+
+
+def test_equal_charges_in_one_cell(cuda):
+    """Four million equal particles in one cell: every rounding of a running FP32 sum then falls the
+    same way. Bar: runs of 16 (8 eps32), a tree of 5, at most 2,048 partial sums one after another
+    (1,024) and the terms' own roundings (8); one sum per lane of a warp is off by 3,300."""
+    torch = cuda
+    from sputnipic_b200 import device
+    wl = W.GemWorkload(name="t", nxc=16, nyc=16, nzc=16, Lx=4.0, Ly=4.0, Lz=4.0)
+    n, q, u = 1 << 22, float(np.float32(0.77)), (0.3, -0.2, 0.1)
+    p = {k: torch.full((n,), 2.125, device="cuda") for k in "xyz"}   # the cell's centre
+    p.update({k: torch.full((n,), a, device="cuda") for k, a in zip("uvw", u)}, q=None)
+    p["q"] = torch.full((n,), q, device="cuda")
+    ctx = device.GridContext(wl)
+    mom = torch.zeros(10, wl.nodes, device="cuda")
+    ctx.p2g(p, mom)
+    assert ctx.check() == 0
+    ctx.close()
+    a, b, c = (float(np.float32(v)) for v in u)
+    want = n * q * 8 * np.array([1, a, b, c, a * a, a * b, a * c, b * b, b * c, c * c])
+    got = mom.double().cpu().numpy().reshape(10, wl.nxn, wl.nyn, wl.nzn)
+    cell = got[:, 9:11, 9:11, 9:11].reshape(10, 8)
+    assert (np.abs(cell / want[:, None] - 1) <= 1042.5 * EPS32).all()
+    assert np.count_nonzero(got) == 80
