@@ -42,6 +42,8 @@ constexpr int SX = TX - 1, SY = TY - 1, SZ = TZ - 1;
 constexpr int TPB = 256;
 // Particles per chunk: bounds the scratch at 2.1 GB of records.
 constexpr long CHUNK_MAX = 1L << 26;
+// Records from which a cell may be summed apart from its tile.
+constexpr int HEAVY_MIN = 1024;
 
 struct Moments10 {
   float *m[10];
@@ -90,12 +92,20 @@ __global__ void __launch_bounds__(TPB) k_p2g_count(GeomDev g, int nty, int ntz,
   }
 }
 
+// Cells with more than `above` records are summed by warps of their own, in
+// segments of about `length` records (k_p2g_cells).
+struct Heavy {
+  unsigned above, length;
+  int4 *segs;   // first record, records, cell key, -
+};
+
 // Every cell's first record: an exclusive scan of the counts inside a CTA, at
-// the place in the record array that the CTA takes for its cells.
+// the place in the record array that the CTA takes for its cells (taken[0]);
+// and the heavy cells' segments (taken[1]: how many).
 constexpr int BASES_TPB = 1024;
 __global__ void __launch_bounds__(BASES_TPB) k_p2g_bases(const unsigned *__restrict__ count,
                                                          long keys, unsigned *__restrict__ first,
-                                                         unsigned *__restrict__ taken) {
+                                                         unsigned *__restrict__ taken, Heavy H) {
   __shared__ unsigned ws[32];
   __shared__ unsigned place;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -120,7 +130,14 @@ __global__ void __launch_bounds__(BASES_TPB) k_p2g_bases(const unsigned *__restr
     if (lane == 31) place = s ? atomicAdd(taken, s) : 0u;
   }
   __syncthreads();
-  if (i < keys) first[i] = place + (warp ? ws[warp - 1] : 0u) + xs - v;
+  const unsigned mine = place + (warp ? ws[warp - 1] : 0u) + xs - v;
+  if (i < keys) first[i] = mine;
+  if (v > H.above) {
+    const unsigned k = (v + H.length - 1) / H.length, len = (v + k - 1) / k;
+    const unsigned at = atomicAdd(taken + 1, k);
+    for (unsigned j = 0, o = 0; j < k; ++j, o = min(o + len, v))
+      H.segs[at + j] = make_int4((int)(mine + o), (int)min(len, v - o), (int)i, 0);
+  }
 }
 
 // Every particle into its cell's next free record (next: the cells' first
@@ -155,33 +172,113 @@ __global__ void __launch_bounds__(TPB) k_p2g_records(GeomDev g, int nty, int ntz
 // the warp's tree they replace.
 constexpr int SUM_RUN = 16;
 
-// One tile of cells (blockIdx.x) and one part of each cell's records
-// (blockIdx.y): thread t sums the records of cell t, the warp those above its
+// The lower nodes' coordinates of a cell and their upper neighbours'.
+struct CellNodes {
+  float2 x, y, z;
+};
+__device__ __forceinline__ CellNodes cell_nodes(const GeomDev &g, int cx, int cy, int cz) {
+  return {__ldg(g.xp + cx + 1), __ldg(g.yp + cy + 1), __ldg(g.zp + cz + 1)};
+}
+
+// Adds record (a, b) to acc (add_terms): a term is f (q xi) eta (zeta invVOL).
+__device__ __forceinline__ void add_record(float2 (&acc)[40], const CellNodes &N, float inv,
+                                           const float4 &a, const float4 &b, int perm) {
+  add_terms(acc, a.w, N.x.y - a.x, a.x - N.x.x, N.y.y - a.y, a.y - N.y.x, (N.z.y - a.z) * inv,
+            (a.z - N.z.x) * inv, b.x, b.y, b.z, perm);
+}
+
+// The heavy cells' segments, one per warp at a time: neighbouring lanes take
+// neighbouring records, and every SUM_RUN of a lane's are summed over the warp
+// into doubles (in shared memory, five per thread: the sums at hand fill the
+// registers).
+__device__ __forceinline__ void sum_segments(const GeomDev &g, int nty, int ntz, int cta, int ctas,
+                                             const unsigned *__restrict__ nsegs,
+                                             const int4 *__restrict__ segs,
+                                             const float4 *__restrict__ recs,
+                                             const Moments10 &M, double *sums) {
+  const int lane = threadIdx.x & 31;
+  const float inv = g.invVOL;
+  const int n = (int)*nsegs;
+  for (int s = cta * (TC / 32) + threadIdx.x / 32; s < n; s += ctas * (TC / 32)) {
+    const int4 seg = segs[s];
+    const int tile = seg.z / TC, c = seg.z % TC;
+    const int cx = tile / (ntz * nty) * TX + c / (TY * TZ) - SX;
+    const int cy = (tile / ntz) % nty * TY + (c / TZ) % TY - SY;
+    const int cz = tile % ntz * TZ + c % TZ - SZ;
+    const CellNodes N = cell_nodes(g, cx, cy, cz);
+    const float4 *rec = recs + 2 * (long)seg.x;
+    double *const sum = sums + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) sum[k * TC] = 0.0;
+    float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na;
+    if (lane < seg.y) ld_rec(rec + 2 * lane, na, nb);
+#pragma unroll 1
+    for (int o = 0; o < seg.y;) {
+      float2 acc[40];
+#pragma unroll
+      for (int i = 0; i < 40; ++i) acc[i] = make_float2(0.f, 0.f);
+      const int stop = min(o + 32 * SUM_RUN, seg.y);
+#pragma unroll 1
+      for (; o < stop; o += 32) {
+        float4 a,b; if (o + lane < seg.y) ld_rec(rec + 2 * (o + lane), a, b);
+        if (o + lane < seg.y) add_record(acc, N, inv, a, b, lane);
+      }
+      float r[5];
+      warp_sum80(acc, r, lane);
+#pragma unroll
+      for (int k = 0; k < 5; ++k) sum[k * TC] += (double)r[k];
+    }
+    const int lo = (lane & 1) ? 3 : 0, hi = (lane & 1) ? 5 : 3, half = (lane >> 1) & 1;
+    const long node = ((long)(cx + ((lane >> 4) & 1)) * g.nyn + (cy + ((lane >> 3) & 1))) * g.nzn +
+                      (cz + ((lane >> 2) & 1));
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+      if (k >= lo && k < hi)
+        atomicAdd((half ? M.m[k + 5] : M.m[k]) + node, (float)(sum[k * TC] * (double)inv));
+  }
+}
+
+// The first CTAs take one tile of cells and one of `parts` parts of each cell's
+// records, the last ones the heavy cells' segments (none on most input: they
+// end as the last tiles are summed). Thread t sums the records of cell t, the warp those above its
 // quota (deposit_quota), and every node of the tile adds its cells' sums into
 // the moments. A term is f (q xi) eta (zeta invVOL),
 // summed in FP32; the second invVOL multiplies a node's sum once (the reference
 // multiplies every term by both): fewer roundings than its own. (q invVOL
 // would round alike for all particles of equal charge: a bias, not noise.)
-__global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, int ntz,
+__global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, int ntz, int tiles,
+                                                            int parts,
                                                             const unsigned *__restrict__ count,
                                                             const unsigned *__restrict__ end,
+                                                            const unsigned *__restrict__ nsegs,
+                                                            Heavy H,
                                                             const float4 *__restrict__ recs,
                                                             const __grid_constant__ Moments10 M) {
   __shared__ float2 sCell[40 * TC];
   const int tid = threadIdx.x, lane = tid & 31;
-  const long key = (long)blockIdx.x * TC + tid;
-  // this CTA's part of the cell's records (gridDim.y parts)
-  const unsigned all = count[key];
-  const unsigned from = (unsigned)((unsigned long long)all * blockIdx.y / gridDim.y);
-  const int cnt = (int)((unsigned)((unsigned long long)all * (blockIdx.y + 1) / gridDim.y) - from);
+  if (blockIdx.x >= tiles * parts) {
+    sum_segments(g, nty, ntz, blockIdx.x - tiles * parts, gridDim.x - tiles * parts,
+                 nsegs, H.segs, recs, M, reinterpret_cast<double *>(sCell));
+    return;
+  }
+  const int part = parts > 1 ? blockIdx.x / tiles : 0, tile = blockIdx.x - part * tiles;
+  const long key = (long)tile * TC + tid;
+  // this CTA's part of the cell's records
+  unsigned all = count[key], from = 0;
+  if (all > H.above) all = 0;
+  int cnt = (int)all;
+  if (parts > 1) {
+    from = (unsigned)((unsigned long long)all * part / parts);
+    cnt = (int)((unsigned)((unsigned long long)all * (part + 1) / parts) - from);
+  }
   if (!__syncthreads_or(cnt)) return;
-  const float4 *rec = recs + 2 * ((long)end[key] - all + from);
-  const int tz = blockIdx.x % ntz, ty = (blockIdx.x / ntz) % nty, tx = blockIdx.x / (ntz * nty);
+  const unsigned rec = end[key] - all + from;   // its first record
+  const int tz = tile % ntz, ty = (tile / ntz) % nty, tx = tile / (ntz * nty);
   // the cell's lower nodes; cells of the tiles off the grid are empty
   const int cx = min(max(tx * TX + tid / (TY * TZ) - SX, 0), g.nxn - 2);
   const int cy = min(max(ty * TY + (tid / TZ) % TY - SY, 0), g.nyn - 2);
   const int cz = min(max(tz * TZ + tid % TZ - SZ, 0), g.nzn - 2);
-  const float2 X = __ldg(g.xp + cx + 1), Y = __ldg(g.yp + cy + 1), Z = __ldg(g.zp + cz + 1);
+  const CellNodes N = cell_nodes(g, cx, cy, cz);
   const float inv = g.invVOL;
   const int Q = deposit_quota(cnt);
   const int n1 = min(cnt, Q);
@@ -190,8 +287,8 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
 #pragma unroll
   for (int i = 0; i < 40; ++i) acc[i] = make_float2(0.f, 0.f);
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, a1 = a, b1 = a;
-  if (n1 > 0) ld_rec(rec, a, b);
-  if (n1 > 1) ld_rec(rec + 2, a1, b1);
+  if (n1 > 0) ld_rec(recs + 2 * (long)rec, a, b);
+  if (n1 > 1) ld_rec(recs + 2 * (long)(rec + 1), a1, b1);
   // the cell's totals take the sums of SUM_RUN particles at a time
   auto put = [&](bool first) {
 #pragma unroll
@@ -204,15 +301,13 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
   for (int k = 0; k < trips; ++k) {
     // two records in flight while this one is summed
     float4 na = a1, nb = b1;
-    if (k + 2 < n1) ld_rec(rec + 2 * (k + 2), na, nb);
+    if (k + 2 < n1) ld_rec(recs + 2 * (long)(rec + k + 2), na, nb);
     // (after the load is on its way: before it, the totals' round through
     // shared memory kept the loads waiting, 55 us of 65.5M particles' 690)
     if (k && k % SUM_RUN == 0) put(k == SUM_RUN);
     // (lanes past their count add nothing: their last record with a charge of
     // zero would turn an infinite product of its velocities into NaN)
-    if (k < n1)
-      add_terms(acc, a.w, X.y - a.x, a.x - X.x, Y.y - a.y, a.y - Y.x, (Z.y - a.z) * inv,
-                (a.z - Z.x) * inv, b.x, b.y, b.z, 0);
+    if (k < n1) add_record(acc, N, inv, a, b, 0);
     a = a1;
     b = b1;
     a1 = na;
@@ -228,11 +323,11 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
       const int hl = __ffs(heavy) - 1;
       heavy &= heavy - 1;
       const int hc = __shfl_sync(FULL, cnt, hl);
-      const float4 *hrec = reinterpret_cast<const float4 *>(
-          __shfl_sync(FULL, reinterpret_cast<unsigned long long>(rec), hl));
-      const float2 hX = make_float2(__shfl_sync(FULL, X.x, hl), __shfl_sync(FULL, X.y, hl));
-      const float2 hY = make_float2(__shfl_sync(FULL, Y.x, hl), __shfl_sync(FULL, Y.y, hl));
-      const float2 hZ = make_float2(__shfl_sync(FULL, Z.x, hl), __shfl_sync(FULL, Z.y, hl));
+      const unsigned hrec = __shfl_sync(FULL, rec, hl);
+      const auto from_hl = [&](float2 v) {
+        return make_float2(__shfl_sync(FULL, v.x, hl), __shfl_sync(FULL, v.y, hl));
+      };
+      const CellNodes hN = {from_hl(N.x), from_hl(N.y), from_hl(N.z)};
       float2 *dst = sCell + corner * 5 * TC + (tid & ~31) + hl;
 #pragma unroll 1
       for (int o = Q; o < hc;) {
@@ -243,9 +338,8 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
         for (; o < stop; o += 32) {
           const int i = o + lane;
           float4 ha = make_float4(0.f, 0.f, 0.f, 0.f), hb = ha;
-          if (i < hc) ld_rec(hrec + 2 * (long)i, ha, hb);
-          add_terms(acc, i < hc ? ha.w : 0.0f, hX.y - ha.x, ha.x - hX.x, hY.y - ha.y,
-                    ha.y - hY.x, (hZ.y - ha.z) * inv, (ha.z - hZ.x) * inv, hb.x, hb.y, hb.z, lane);
+          if (i < hc) ld_rec(recs + 2 * (long)(hrec + i), ha, hb);
+          add_record(acc, hN, inv, ha, hb, lane);
         }
         float r[5];
         warp_sum80(acc, r, lane);
@@ -278,13 +372,16 @@ int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z,
             ntz = (int)ceil_div(g.nzn - 1 + SZ, TZ);
   const long tiles = (long)ntx * nty * ntz, keys = tiles * TC;
   if (keys >= (1L << 31)) return SPB_OK;   // cell keys are ints: not in cell order
-  // records of a chunk, the cells' counts and a counter, the cells' places;
-  // chunks are halved until their scratch can be had
+  // records of a chunk, the heavy cells' segments (at most one per HEAVY_MIN
+  // particles), the cells' counts and two counters, the cells' places; chunks
+  // are halved until their scratch can be had
   long chunk = ceil_div(n, ceil_div(n, CHUNK_MAX));
   unsigned char *scratch = nullptr;
   for (;; chunk = ceil_div(chunk, 2)) {
     scratch = static_cast<unsigned char *>(
-        pool_alloc((size_t)chunk * 32 + (size_t)(2 * keys + 1) * sizeof(unsigned), s));
+        pool_alloc((size_t)chunk * 32 + (size_t)(chunk / HEAVY_MIN + 1) * sizeof(int4) +
+                       (size_t)(2 * keys + 2) * sizeof(unsigned),
+                   s));
     if (scratch && (reinterpret_cast<uintptr_t>(scratch) & 31u)) {   // records are 32-byte accesses
       pool_free(scratch, s);
       scratch = nullptr;
@@ -293,8 +390,9 @@ int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z,
     if (chunk < 2 * SORTED_P2G_MIN) return SPB_OK;
   }
   float4 *rec = reinterpret_cast<float4 *>(scratch);
-  unsigned *count = reinterpret_cast<unsigned *>(scratch + (size_t)chunk * 32);
-  unsigned *taken = count + keys, *next = taken + 1;
+  int4 *segs = reinterpret_cast<int4 *>(scratch + (size_t)chunk * 32);
+  unsigned *count = reinterpret_cast<unsigned *>(segs + chunk / HEAVY_MIN + 1);
+  unsigned *taken = count + keys, *next = taken + 2;
   Moments10 M;
   for (int m = 0; m < 10; ++m) M.m[m] = mom[m];
   // on small grids the cells' records go to several CTAs: a thread walks its
@@ -304,22 +402,32 @@ int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z,
   const long inner = std::max(1L, ceil_div(g.nxn - 3, TX)) *
                      std::max(1L, ceil_div(g.nyn - 3, TY)) *
                      std::max(1L, ceil_div(g.nzn - 3, TZ));
-  const unsigned parts = (unsigned)std::max(
-      1L, std::min({4L, 4L * num_sms() / inner, chunk / (8 * inner * TC)}));
+  const int places = 4 * num_sms();
+  const int parts = (int)std::max(1L, std::min(places / inner, chunk / (8 * inner * TC)));
+  // heavy cells: more than eight times the mean of the inner tiles' cells, so
+  // that none keeps its tile much longer than the others keep theirs; their
+  // segments are as long as leaves every warp of the launch one. 4x4x4 cells with
+  // 10M particles 0.63 ms, 23.8 with at most four parts; 128x64x64 cells with 20M
+  // of which a third in one cell 1.04 ms, 121 if a warp walks that cell, all in
+  // one cell 1.35 ms, 4.6 s
+  const Heavy H{(unsigned)std::max<long>(HEAVY_MIN, chunk / (inner * (TC / 8))),
+                (unsigned)std::max(2L * HEAVY_MIN, ceil_div(chunk, (long)places * (TC / 32))),
+                segs};
   int rc = SPB_OK;
   for (long off = 0; off < n && rc == SPB_OK; off += chunk) {
     const long c = std::min(chunk, n - off);
     const unsigned blocks = (unsigned)std::min<long>(ceil_div(c, TPB), 148L * 32);
     const Particles7 P{{x + off, y + off, z + off, u + off, v + off, w + off, q + off}};
-    cudaError_t e = cudaMemsetAsync(count, 0, (size_t)(keys + 1) * sizeof(unsigned), s);
+    cudaError_t e = cudaMemsetAsync(count, 0, (size_t)(keys + 2) * sizeof(unsigned), s);
     if (e == cudaSuccess) {
       (g.float_cells ? k_p2g_count<true> : k_p2g_count<false>)<<<blocks, TPB, 0, s>>>(
           g, nty, ntz, P.p[0], P.p[1], P.p[2], c, count);
       k_p2g_bases<<<(unsigned)ceil_div(keys, BASES_TPB), BASES_TPB, 0, s>>>(count, keys, next,
-                                                                            taken);
+                                                                            taken, H);
       (g.float_cells ? k_p2g_records<true> : k_p2g_records<false>)<<<blocks, TPB, 0, s>>>(
           g, nty, ntz, P, c, next, rec, err);
-      k_p2g_cells<<<dim3((unsigned)tiles, parts), TC, 0, s>>>(g, nty, ntz, count, next, rec, M);
+      k_p2g_cells<<<(unsigned)(tiles * parts + places), TC, 0, s>>>(
+          g, nty, ntz, (int)tiles, parts, count, next, taken + 1, H, rec, M);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) rc = fail_cuda(e, "sorted_p2g");

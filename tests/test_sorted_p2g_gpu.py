@@ -167,3 +167,49 @@ def test_equal_charges_in_one_cell(cuda):
     cell = got[:, 9:11, 9:11, 9:11].reshape(10, 8)
     assert (np.abs(cell / want[:, None] - 1) <= 1042.5 * EPS32).all()
     assert np.count_nonzero(got) == 80
+
+
+def check64(got, wl, p, bar):
+    """|gpu - FP64| <= bar eps32 sum |term| per node."""
+    setup = oracle.setup_from(wl)
+    o64 = oracle.CpuOracle("restated", 64)
+    ref, absm = ([np.zeros(wl.nodes) for _ in range(10)] for _ in range(2))
+    d = {k: p[k].astype(np.float64) for k in "xyzuvwq"}
+    o64.interp_p2g(setup, d, ref)
+    o64.interp_p2g(setup, {k: (np.abs(v) if k in "uvwq" else v) for k, v in d.items()}, absm)
+    err = np.abs(got.astype(np.float64) - np.stack(ref))
+    worst = (err / (EPS32 * np.stack(absm) + 1e-30)).max()
+    assert worst <= bar, worst
+
+
+@pytest.mark.parametrize("grid", [(1, 1, 1), (4, 4, 4), (1, 1, 300), (40, 24, 16)])
+@pytest.mark.parametrize("where", ["anywhere", "a third in one cell", "one cell", "sizes"])
+def test_clumps_and_tiny_grids(cuda, grid, where):
+    """Millions of particles on few cells, or in one cell of many, and cells at the counts where the
+    split of their records changes. Cells are 1/4 wide, so node distances are exact; a term has at
+    most 8 roundings, a sum runs of 16 and a tree of 5 (random ones: under 8 eps32), and a node at
+    most 2,400 FP32 adds of partial sums, random in sign: 0.29 sqrt(2400 / 3) < 9 eps32."""
+    torch = cuda
+    from sputnipic_b200 import device
+    rng = np.random.default_rng(sum(grid))
+    wl = W.GemWorkload(name="t", nxc=grid[0], nyc=grid[1], nzc=grid[2], Lx=grid[0] * 0.25,
+                       Ly=grid[1] * 0.25, Lz=grid[2] * 0.25)
+    n = (1 << 21) + 5
+    p = particles(rng, wl, n, "anywhere")
+    held = {"a third in one cell": [n // 3], "one cell": [n],
+            "sizes": [1023, 1024, 1025, 2047, 2048, 2049, 4097, 100_000, 300_001]}.get(where, [])
+    at = 0
+    for m in held:
+        for k, c in zip("xyz", grid):
+            p[k][at:at + m] = (rng.integers(0, c) + rng.random(m)).astype(np.float32) * 0.25
+        at += m
+    for k, L in zip("xyz", (wl.Lx, wl.Ly, wl.Lz)):
+        p[k] = np.minimum(p[k], np.nextafter(np.float32(L), np.float32(0)))
+    order = rng.permutation(n)
+    p = {k: v[order] for k, v in p.items()}
+    ctx = device.GridContext(wl)
+    mom = torch.zeros(10, wl.nodes, device="cuda")
+    ctx.p2g(on_gpu(torch, p), mom)
+    assert ctx.check() == 0
+    check64(mom.cpu().numpy(), wl, p, 32)
+    ctx.close()
