@@ -213,3 +213,34 @@ def test_clumps_and_tiny_grids(cuda, grid, where):
     assert ctx.check() == 0
     check64(mom.cpu().numpy(), wl, p, 32)
     ctx.close()
+
+
+@pytest.mark.parametrize("busy", [1, 31, 32, 33, 128])
+@pytest.mark.parametrize("most", [1, 16, 17])
+def test_sparse_tiles(cuda, busy, most):
+    """Tiles with few cells that hold particles, and few particles in each, on both sides of the
+    counts from which their cells' sums go through the node sums."""
+    torch = cuda
+    from sputnipic_b200 import device
+    rng = np.random.default_rng(busy)
+    wl = W.GemWorkload(name="t", nxc=80, nyc=40, nzc=40, Lx=20.0, Ly=10.0, Lz=10.0)
+    cells = np.indices((80, 40, 40)).reshape(3, -1).T.reshape(10, 8, 10, 4, 10, 4, 3)
+    tiles = cells.transpose(0, 2, 4, 1, 3, 5, 6).reshape(1000, 128, 3)
+    at = np.concatenate([t[rng.permutation(128)[:busy]] for t in tiles])
+    count = rng.integers(1, most + 1, len(at))
+    count[0] = most
+    at = np.repeat(at, count, axis=0)
+    lone = 65_536 - len(at)   # a first inner tile with everything that is missing
+    if lone > 0:
+        at = np.concatenate([at, tiles[0][rng.integers(0, 128, lone)]])
+    p = {k: ((at[:, a] + rng.uniform(0, 0.999, len(at))) * 0.25).astype(np.float32)
+         for a, k in enumerate("xyz")}
+    for k in "uvw":
+        p[k] = (0.05 * rng.standard_normal(len(at))).astype(np.float32)
+    p["q"] = rng.uniform(-1, 1, len(at)).astype(np.float32)
+    ctx = device.GridContext(wl)
+    mom = torch.zeros(10, wl.nodes, device="cuda")
+    ctx.p2g(on_gpu(torch, p), mom)
+    assert ctx.check() == 0
+    check(mom.cpu().numpy(), wl, p)
+    ctx.close()
