@@ -17,12 +17,12 @@
 // applyBCids included: 2352 -> 1455 us (count 150, copy 680, sum 600); two
 // species of 2.4M some cycles after the last sort, 27 per cell: 432 -> 232 us.
 //
-// Cells are numbered tile by tile (8 x 4 x 4 cells; a CTA of the last launch
-// takes a tile), over the nxn - 1 cells per axis that node pairs (i - 1, i)
-// span, guard cells included. The first inner cell starts a tile, so that on a
-// grid of whole tiles the guard cells, empty but for particles on a wall, fill
-// tiles of their own, which end at once (the GEM grid: 4096 tiles of full cells
-// instead of 4913 of which 817 held one layer).
+// Cells are numbered tile by tile (8 x 4 x 4 cells, on thin grids of one layer;
+// a CTA of the last launch takes a tile), over the nxn - 1 cells per axis that
+// node pairs (i - 1, i) span, guard cells included. The first inner cell starts a
+// tile, so that on a grid of whole tiles the guard cells, empty but for particles
+// on a wall, fill tiles of their own, which end at once (the GEM grid: 4096 tiles
+// of full cells instead of 4913 of which 817 held one layer).
 #include "cell_deposit.cuh"
 #include "grid_ctx.h"
 #include "kernels.h"
@@ -36,9 +36,7 @@ namespace spb {
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int TX = 8, TY = 4, TZ = 4, TC = TX * TY * TZ;
-// Positions that cell 0, the lower guard cell, lies into its tile.
-constexpr int SX = TX - 1, SY = TY - 1, SZ = TZ - 1;
+constexpr int TC = 128;   // cells of a tile, TX x TY x TZ
 constexpr int TPB = 256;
 // Particles per chunk: bounds the scratch at 2.1 GB of records.
 constexpr long CHUNK_MAX = 1L << 26;
@@ -53,17 +51,18 @@ struct Particles7 {
   const float *p[7];   // x, y, z, u, v, w, q
 };
 
-// The deposit cell of a particle, as a key.
-template <bool FLOAT_CELLS>
+// The deposit cell of a particle, as a key (cell 0 of an axis, the lower guard
+// cell, is its tile's last).
+template <int TX, int TY, int TZ, bool FLOAT_CELLS>
 __device__ __forceinline__ int cell_key(const GeomDev &g, int nty, int ntz, float x, float y,
                                         float z, int &bad) {
   int ix, iy, iz;
   deposit_cell<FLOAT_CELLS>(g, x, y, z, ix, iy, iz, bad);
-  return tile_key<TX, TY, TZ>(ix - 1 + SX, iy - 1 + SY, iz - 1 + SZ, nty, ntz);
+  return tile_key<TX, TY, TZ>(ix + TX - 2, iy + TY - 2, iz + TZ - 2, nty, ntz);
 }
 
 // Particles per cell (one atomic per distinct cell of a warp).
-template <bool FLOAT_CELLS>
+template <int TX, int TY, int TZ, bool FLOAT_CELLS>
 __global__ void __launch_bounds__(TPB) k_p2g_count(GeomDev g, int nty, int ntz,
                                                    const float *__restrict__ x,
                                                    const float *__restrict__ y,
@@ -85,7 +84,8 @@ __global__ void __launch_bounds__(TPB) k_p2g_count(GeomDev g, int nty, int ntz,
     for (int k = 0; k < U; ++k) {
       const bool valid = base + k * TPB + threadIdx.x < n;
       const int key =
-          valid ? cell_key<FLOAT_CELLS>(g, nty, ntz, p[k][0], p[k][1], p[k][2], ignored) : -1;
+          valid ? cell_key<TX, TY, TZ, FLOAT_CELLS>(g, nty, ntz, p[k][0], p[k][1], p[k][2], ignored)
+                : -1;
       const unsigned peers = __match_any_sync(FULL, key);
       if (valid && lane == __ffs(peers) - 1) atomicAdd(count + key, (unsigned)__popc(peers));
     }
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(BASES_TPB) k_p2g_bases(const unsigned *__restr
 
 // Every particle into its cell's next free record (next: the cells' first
 // records, advanced to their ends; the order inside a cell is the atomics').
-template <bool FLOAT_CELLS>
+template <int TX, int TY, int TZ, bool FLOAT_CELLS>
 __global__ void __launch_bounds__(TPB) k_p2g_records(GeomDev g, int nty, int ntz,
                                                      const __grid_constant__ Particles7 P, long n,
                                                      unsigned *__restrict__ next,
@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(TPB) k_p2g_records(GeomDev g, int nty, int ntz
     const long i = valid ? base + threadIdx.x : n - 1;   // every lane loads: no branch
     const float4 a = make_float4(P.p[0][i], P.p[1][i], P.p[2][i], P.p[6][i]);
     const float4 b = make_float4(P.p[3][i], P.p[4][i], P.p[5][i], 0.f);
-    const int key = valid ? cell_key<FLOAT_CELLS>(g, nty, ntz, a.x, a.y, a.z, bad) : -1;
+    const int key =
+        valid ? cell_key<TX, TY, TZ, FLOAT_CELLS>(g, nty, ntz, a.x, a.y, a.z, bad) : -1;
     const unsigned peers = __match_any_sync(FULL, key);
     const int leader = __ffs(peers) - 1;
     unsigned at = 0;
@@ -197,6 +198,7 @@ __device__ __forceinline__ void add_record(float2 (&acc)[40], const CellNodes &N
 // neighbouring records, and every SUM_RUN of a lane's are summed over the warp
 // into doubles (in shared memory, five per thread: the sums at hand fill the
 // registers).
+template <int TX, int TY, int TZ>
 __device__ __forceinline__ void sum_segments(const GeomDev &g, int nty, int ntz, int cta, int ctas,
                                              const unsigned *__restrict__ nsegs,
                                              const int4 *__restrict__ segs,
@@ -208,9 +210,9 @@ __device__ __forceinline__ void sum_segments(const GeomDev &g, int nty, int ntz,
   for (int s = cta * (TC / 32) + threadIdx.x / 32; s < n; s += ctas * (TC / 32)) {
     const int4 seg = segs[s];
     const int tile = seg.z / TC, c = seg.z % TC;
-    const int cx = tile / (ntz * nty) * TX + c / (TY * TZ) - SX;
-    const int cy = (tile / ntz) % nty * TY + (c / TZ) % TY - SY;
-    const int cz = tile % ntz * TZ + c % TZ - SZ;
+    const int cx = tile / (ntz * nty) * TX + c / (TY * TZ) - (TX - 1);
+    const int cy = (tile / ntz) % nty * TY + (c / TZ) % TY - (TY - 1);
+    const int cz = tile % ntz * TZ + c % TZ - (TZ - 1);
     const CellNodes N = cell_nodes(g, cx, cy, cz);
     const float4 *rec = recs + 2 * (long)seg.x;
     double *const sum = sums + threadIdx.x;
@@ -277,6 +279,7 @@ __device__ __forceinline__ void add_cell(const GeomDev &g, const CellNodes &N, i
 // summed in FP32; the second invVOL multiplies a node's sum once (the reference
 // multiplies every term by both): fewer roundings than its own. (q invVOL
 // would round alike for all particles of equal charge: a bias, not noise.)
+template <int TX, int TY, int TZ>
 __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, int ntz, int tiles,
                                                             int parts,
                                                             const unsigned *__restrict__ count,
@@ -288,8 +291,8 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
   __shared__ float2 sCell[40 * TC];
   const int tid = threadIdx.x, lane = tid & 31;
   if (blockIdx.x >= tiles * parts) {
-    sum_segments(g, nty, ntz, blockIdx.x - tiles * parts, gridDim.x - tiles * parts,
-                 nsegs, H.segs, recs, M, reinterpret_cast<double *>(sCell));
+    sum_segments<TX, TY, TZ>(g, nty, ntz, blockIdx.x - tiles * parts, gridDim.x - tiles * parts,
+                             nsegs, H.segs, recs, M, reinterpret_cast<double *>(sCell));
     return;
   }
   const int part = parts > 1 ? blockIdx.x / tiles : 0, tile = blockIdx.x - part * tiles;
@@ -307,9 +310,9 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
   const unsigned rec = end[key] - all + from;   // its first record
   const int tz = tile % ntz, ty = (tile / ntz) % nty, tx = tile / (ntz * nty);
   // the cell's lower nodes; cells of the tiles off the grid are empty
-  const int cx = min(max(tx * TX + tid / (TY * TZ) - SX, 0), g.nxn - 2);
-  const int cy = min(max(ty * TY + (tid / TZ) % TY - SY, 0), g.nyn - 2);
-  const int cz = min(max(tz * TZ + tid % TZ - SZ, 0), g.nzn - 2);
+  const int cx = min(max(tx * TX + tid / (TY * TZ) - (TX - 1), 0), g.nxn - 2);
+  const int cy = min(max(ty * TY + (tid / TZ) % TY - (TY - 1), 0), g.nyn - 2);
+  const int cz = min(max(tz * TZ + tid % TZ - (TZ - 1), 0), g.nzn - 2);
   const CellNodes N = cell_nodes(g, cx, cy, cz);
   const float inv = g.invVOL;
   if (busy <= SPARSE_CELLS && !__syncthreads_or(cnt > SUM_RUN)) {
@@ -388,8 +391,8 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
   __syncthreads();
   node_sums<TX, TY, TZ, TC, float, double>(sCell, [&](int bx, int by, int bz,
                                                       const double2(&sum)[5]) {
-    const long n = ((long)(tx * TX + bx - SX) * g.nyn + (ty * TY + by - SY)) * g.nzn +
-                   (tz * TZ + bz - SZ);
+    const long n = ((long)(tx * TX + bx - (TX - 1)) * g.nyn + (ty * TY + by - (TY - 1))) * g.nzn +
+                   (tz * TZ + bz - (TZ - 1));
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       if (sum[k].x != 0.0) atomicAdd(M.m[k] + n, (float)(sum[k].x * (double)inv));
@@ -398,14 +401,20 @@ __global__ void __launch_bounds__(TC, 512 / TC) k_p2g_cells(GeomDev g, int nty, 
   });
 }
 
-}  // namespace
+// Tiles of TX x TY x TZ cells that hold inner cells.
+template <int TX, int TY, int TZ>
+long inner_tiles(const GeomDev &g) {
+  return std::max(1L, ceil_div(g.nxn - 3, TX)) * std::max(1L, ceil_div(g.nyn - 3, TY)) *
+         std::max(1L, ceil_div(g.nzn - 3, TZ));
+}
 
-int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z, const float *u,
+template <int TX, int TY, int TZ>
+int sorted_p2g_by(const GeomDev &g, const float *x, const float *y, const float *z, const float *u,
                const float *v, const float *w, const float *q, long n, float *const mom[10],
                int *err, cudaStream_t s, long *done) {
   *done = 0;
-  const int ntx = (int)ceil_div(g.nxn - 1 + SX, TX), nty = (int)ceil_div(g.nyn - 1 + SY, TY),
-            ntz = (int)ceil_div(g.nzn - 1 + SZ, TZ);
+  const int ntx = (int)ceil_div(g.nxn + TX - 2, TX), nty = (int)ceil_div(g.nyn + TY - 2, TY),
+            ntz = (int)ceil_div(g.nzn + TZ - 2, TZ);
   const long tiles = (long)ntx * nty * ntz, keys = tiles * TC;
   if (keys >= (1L << 31)) return SPB_OK;   // cell keys are ints: not in cell order
   // records of a chunk, the heavy cells' segments (at most one per HEAVY_MIN
@@ -435,9 +444,7 @@ int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z,
   // cell's one after another, and with fewer tiles than CTAs fit (four per SM)
   // that walk is the launch's time; parts of at least eight records a cell
   // (32x16x16 cells at 27 per cell: 22 -> 13 us)
-  const long inner = std::max(1L, ceil_div(g.nxn - 3, TX)) *
-                     std::max(1L, ceil_div(g.nyn - 3, TY)) *
-                     std::max(1L, ceil_div(g.nzn - 3, TZ));
+  const long inner = inner_tiles<TX, TY, TZ>(g);
   const int places = 4 * num_sms();
   const int parts = (int)std::max(1L, std::min(places / inner, chunk / (8 * inner * TC)));
   // heavy cells: more than eight times the mean of the inner tiles' cells, so
@@ -456,13 +463,15 @@ int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z,
     const Particles7 P{{x + off, y + off, z + off, u + off, v + off, w + off, q + off}};
     cudaError_t e = cudaMemsetAsync(count, 0, (size_t)(keys + 2) * sizeof(unsigned), s);
     if (e == cudaSuccess) {
-      (g.float_cells ? k_p2g_count<true> : k_p2g_count<false>)<<<blocks, TPB, 0, s>>>(
-          g, nty, ntz, P.p[0], P.p[1], P.p[2], c, count);
+      auto *const k_count = g.float_cells ? k_p2g_count<TX, TY, TZ, true>
+                                          : k_p2g_count<TX, TY, TZ, false>;
+      auto *const k_records = g.float_cells ? k_p2g_records<TX, TY, TZ, true>
+                                            : k_p2g_records<TX, TY, TZ, false>;
+      k_count<<<blocks, TPB, 0, s>>>(g, nty, ntz, P.p[0], P.p[1], P.p[2], c, count);
       k_p2g_bases<<<(unsigned)ceil_div(keys, BASES_TPB), BASES_TPB, 0, s>>>(count, keys, next,
                                                                             taken, H);
-      (g.float_cells ? k_p2g_records<true> : k_p2g_records<false>)<<<blocks, TPB, 0, s>>>(
-          g, nty, ntz, P, c, next, rec, err);
-      k_p2g_cells<<<(unsigned)(tiles * parts + places), TC, 0, s>>>(
+      k_records<<<blocks, TPB, 0, s>>>(g, nty, ntz, P, c, next, rec, err);
+      k_p2g_cells<TX, TY, TZ><<<(unsigned)(tiles * parts + places), TC, 0, s>>>(
           g, nty, ntz, (int)tiles, parts, count, next, taken + 1, H, rec, M);
       e = cudaGetLastError();
     }
@@ -472,6 +481,25 @@ int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z,
   pool_free(scratch, s);
   if (rc == SPB_OK) *done = n;
   return rc;
+}
+
+}  // namespace
+
+int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z, const float *u,
+               const float *v, const float *w, const float *q, long n, float *const mom[10],
+               int *err, cudaStream_t s, long *done) {
+  // on grids a few cells thin, tiles of one layer along that axis, where they
+  // hold the cells in two thirds of the tiles or fewer (a layer's tile has 306
+  // nodes to sum, not 225). 10M particles, 512x512x1 cells: 557 -> 321 us;
+  // 1x512x512: 978 -> 316
+  const auto pick = [&]() -> decltype(&sorted_p2g_by<8, 4, 4>) {
+    const long most = 2 * inner_tiles<8, 4, 4>(g) / 3;
+    if (inner_tiles<1, 16, 8>(g) <= most) return sorted_p2g_by<1, 16, 8>;
+    if (inner_tiles<8, 1, 16>(g) <= most) return sorted_p2g_by<8, 1, 16>;
+    if (inner_tiles<8, 16, 1>(g) <= most) return sorted_p2g_by<8, 16, 1>;
+    return sorted_p2g_by<8, 4, 4>;
+  };
+  return pick()(g, x, y, z, u, v, w, q, n, mom, err, s, done);
 }
 
 }  // namespace spb

@@ -244,3 +244,21 @@ def test_sparse_tiles(cuda, busy, most):
     assert ctx.check() == 0
     check(mom.cpu().numpy(), wl, p)
     ctx.close()
+
+
+@pytest.mark.parametrize("grid", [(1, 40, 33), (2, 31, 64), (40, 1, 33), (33, 2, 40), (40, 33, 1),
+                                  (31, 64, 2), (3, 20, 20), (4, 40, 40)])
+@pytest.mark.parametrize("where", ["anywhere", "one cell", "nodes"])
+def test_thin_grids(cuda, grid, where):
+    """Grids a few cells thin along each axis: the tiles of one layer, and those next to the rule."""
+    torch = cuda
+    from sputnipic_b200 import device
+    wl = W.GemWorkload(name="t", nxc=grid[0], nyc=grid[1], nzc=grid[2], Lx=grid[0] * 0.25,
+                       Ly=grid[1] * 0.25, Lz=grid[2] * 0.25)
+    p = particles(np.random.default_rng(sum(grid)), wl, 70_001, where)
+    ctx = device.GridContext(wl)
+    mom = torch.zeros(10, wl.nodes, device="cuda")
+    ctx.p2g(on_gpu(torch, p), mom)
+    assert ctx.check() == 0
+    check(mom.cpu().numpy(), wl, p)
+    ctx.close()
