@@ -331,13 +331,9 @@ int run_copy_pipelined(Op op, Species *sp, struct particles *part, struct EMfiel
       if (!f[a]) return fail(SPB_ERR_INVALID, "field array is null");
     if (int rc = spb_grid_set_fields(ctx, f, 0, sp->stream)) return rc;
   }
-  float *acc = nullptr;   // the last chunk's accumulator
-  if (deposits) {
+  float *acc[NPIPE] = {};   // accumulators of the chunks that are not deposited in cell order
+  if (deposits)
     if (int rc = upload_moments(sp, ids, nodes, dev_mom, hm, dm)) return rc;
-    // only a last chunk too small for the sorted deposit adds into one
-    if (n % PIPE_CHUNK && plain_wants_acc(n % PIPE_CHUNK))
-      acc = plain_acc_alloc(ctx->geom, sp->stream);
-  }
   SPB_CUDA(cudaEventRecord(sp->ev_in, sp->stream));
   for (int j = 0; j < NPIPE; ++j) SPB_CUDA(cudaStreamWaitEvent(sp->pipe[j], sp->ev_in, 0));
   const PushDev p = moves ? make_push(push_of(part, param)) : PushDev{};
@@ -354,18 +350,15 @@ int run_copy_pipelined(Op op, Species *sp, struct particles *part, struct EMfiel
     int rc;
     if (op == Op::Fused)
       rc = launch_plain_mover_interp_into(ctx->geom, p, F, d[0], d[1], d[2], d[3], d[4], d[5],
-                                          d[6], cnt, acc, dm, sp->d_err, s);
+                                          d[6], cnt, &acc[k % NPIPE], dm, sp->d_err, s);
     else if (moves)
       rc = launch_plain_mover(ctx->geom, p, F, d[0], d[1], d[2], d[3], d[4], d[5], cnt,
                               sp->d_err, s, op == Op::MoverV ? 1 : 0);
     else
-      rc = launch_plain_p2g_into(ctx->geom, d[0], d[1], d[2], d[3], d[4], d[5], d[6], cnt, acc,
-                                 dm, sp->d_err, s);
+      rc = launch_plain_p2g_into(ctx->geom, d[0], d[1], d[2], d[3], d[4], d[5], d[6], cnt,
+                                 &acc[k % NPIPE], dm, sp->d_err, s);
     if (rc) {
-      if (acc) {   // after the chunks already queued on the pipe streams
-        for (int j = 0; j < NPIPE; ++j) cudaStreamSynchronize(sp->pipe[j]);
-        cudaFreeAsync(acc, sp->stream);
-      }
+      for (int j = 0; j < NPIPE; ++j) pool_free(acc[j], sp->pipe[j]);
       return rc;
     }
     ctx->launches++;
@@ -377,10 +370,11 @@ int run_copy_pipelined(Op op, Species *sp, struct particles *part, struct EMfiel
     SPB_CUDA(cudaEventRecord(sp->ev_done[j], sp->pipe[j]));
     SPB_CUDA(cudaStreamWaitEvent(sp->stream, sp->ev_done[j], 0));
   }
-  if (acc) {
-    if (int rc = plain_acc_fold(acc, ctx->geom, dm, sp->stream)) return rc;
-    ctx->launches++;
-  }
+  for (int j = 0; j < NPIPE; ++j)
+    if (acc[j]) {
+      if (int rc = plain_acc_fold(acc[j], ctx->geom, dm, sp->stream)) return rc;
+      ctx->launches++;
+    }
   if (deposits && !dev_mom)
     for (int m = 0; m < 10; ++m)
       SPB_CUDA(cudaMemcpyAsync(hm[m], dm[m], nodes * sizeof(float), cudaMemcpyDeviceToHost,

@@ -37,9 +37,6 @@ void pool_free(void *p, cudaStream_t s);
 // stream-ordered pool on stream s, or nullptr when it cannot be had (the
 // deposits then add straight into the moment arrays).
 float *plain_acc_alloc(const GeomDev &g, cudaStream_t s);
-// Whether a deposit of n particles adds into an accumulator (the others go
-// through sorted_p2g straight into the moment arrays).
-bool plain_wants_acc(long n);
 // Adds the accumulator into mom[0..9] and returns it to the pool (nothing
 // for nullptr).
 int plain_acc_fold(float *acc, const GeomDev &g, float *const mom[10], cudaStream_t s);
@@ -50,13 +47,15 @@ constexpr long SORTED_P2G_MIN = 65536;
 int sorted_p2g(const GeomDev &g, const float *x, const float *y, const float *z, const float *u,
                const float *v, const float *w, const float *q, long n, float *const mom[10],
                int *err, cudaStream_t s, long *done);
-// interpP2G / mover_interp deposits into acc (mom when acc is nullptr).
+// interpP2G / mover_interp deposits: what is not deposited in cell order goes
+// into *acc, allocated on s when first needed (mom where it cannot be had).
+// The caller folds it, or returns it to the pool after an error.
 int launch_plain_p2g_into(const GeomDev &g, const float *x, const float *y, const float *z,
                           const float *u, const float *v, const float *w, const float *q, long n,
-                          float *acc, float *const mom[10], int *err, cudaStream_t s);
+                          float **acc, float *const mom[10], int *err, cudaStream_t s);
 int launch_plain_mover_interp_into(const GeomDev &g, const PushDev &p, const PackedFields &F,
                                    float *x, float *y, float *z, float *u, float *v, float *w,
-                                   const float *q, long n, float *acc, float *const mom[10],
+                                   const float *q, long n, float **acc, float *const mom[10],
                                    int *err, cudaStream_t s);
 // The same with their own accumulator: allocate, deposit, fold.
 int launch_plain_p2g(const GeomDev &g, const float *x, const float *y, const float *z,

@@ -840,15 +840,16 @@ DepTarget target(float *acc, float *const mom[10]) {
 
 int launch_plain_p2g_into(const GeomDev &g, const float *x, const float *y, const float *z,
                           const float *u, const float *v, const float *w, const float *q, long n,
-                          float *acc, float *const mom[10], int *err, cudaStream_t s) {
+                          float **acc, float *const mom[10], int *err, cudaStream_t s) {
   if (n <= 0) return SPB_OK;
   long done = 0;   // particles deposited in cell order
   if (n >= P2S_MIN)
     if (int rc = sorted_p2g(g, x, y, z, u, v, w, q, n, mom, err, s, &done)) return rc;
   if (done == n) return SPB_OK;
-  const DepTarget T = target(acc, mom);
+  if (!*acc) *acc = plain_acc_alloc(g, s);
+  const DepTarget T = target(*acc, mom);
   const unsigned chunks = (unsigned)ceil_div(n - done, GP_CHUNK);
-  auto *const kernel = acc ? k_plain_p2g_grouped<true> : k_plain_p2g_grouped<false>;
+  auto *const kernel = *acc ? k_plain_p2g_grouped<true> : k_plain_p2g_grouped<false>;
   kernel<<<chunks, GP_TPB, 0, s>>>(g, x + done, y + done, z + done, u + done, v + done, w + done,
                                    q + done, n - done, T, err);
   SPB_CUDA(cudaGetLastError());
@@ -858,20 +859,18 @@ int launch_plain_p2g_into(const GeomDev &g, const float *x, const float *y, cons
 
 int launch_plain_mover_interp_into(const GeomDev &g, const PushDev &p, const PackedFields &F,
                                    float *x, float *y, float *z, float *u, float *v, float *w,
-                                   const float *q, long n, float *acc, float *const mom[10],
+                                   const float *q, long n, float **acc, float *const mom[10],
                                    int *err, cudaStream_t s) {
   if (int rc = launch_plain_mover(g, p, F, x, y, z, u, v, w, n, err, s)) return rc;
   return launch_plain_p2g_into(g, x, y, z, u, v, w, q, n, acc, mom, err, s);
 }
 
-bool plain_wants_acc(long n) { return n < P2S_MIN; }
-
 int launch_plain_p2g(const GeomDev &g, const float *x, const float *y, const float *z,
                      const float *u, const float *v, const float *w, const float *q, long n,
                      float *const mom[10], int *err, cudaStream_t s) {
   if (n <= 0) return SPB_OK;
-  float *acc = plain_wants_acc(n) ? plain_acc_alloc(g, s) : nullptr;
-  const int rc = launch_plain_p2g_into(g, x, y, z, u, v, w, q, n, acc, mom, err, s);
+  float *acc = nullptr;
+  const int rc = launch_plain_p2g_into(g, x, y, z, u, v, w, q, n, &acc, mom, err, s);
   if (rc) {
     if (acc) cudaFreeAsync(acc, s);
     return rc;

@@ -262,3 +262,109 @@ def test_thin_grids(cuda, grid, where):
     assert ctx.check() == 0
     check(mom.cpu().numpy(), wl, p)
     ctx.close()
+
+
+@pytest.fixture
+def small_pool(cuda):
+    """The device's memory pool replaced by one of 32 MB, of which `held` bytes are taken."""
+    from contextlib import contextmanager
+
+    from cuda.bindings import runtime as rt
+
+    def ok(r):
+        assert int(r[0]) == 0, r[0]
+        return r[1] if len(r) > 1 else None
+
+    @contextmanager
+    def replaced(held):
+        props = rt.cudaMemPoolProps()
+        props.allocType = rt.cudaMemAllocationType.cudaMemAllocationTypePinned
+        props.location.type = rt.cudaMemLocationType.cudaMemLocationTypeDevice
+        props.location.id = 0
+        props.maxSize = 32 << 20
+        cuda.cuda.synchronize()
+        pool = ok(rt.cudaMemPoolCreate(props))
+        taken = ok(rt.cudaMallocFromPoolAsync(held, pool, 0)) if held else None
+        ok(rt.cudaDeviceSetMemPool(0, pool))
+        try:
+            yield
+        finally:
+            cuda.cuda.synchronize()
+            ok(rt.cudaDeviceSetMemPool(0, ok(rt.cudaDeviceGetDefaultMemPool(0))))
+            if taken is not None:
+                ok(rt.cudaFreeAsync(taken, 0))
+            cuda.cuda.synchronize()
+            ok(rt.cudaMemPoolDestroy(pool))
+    return replaced
+
+
+@pytest.fixture(params=["accumulator", "direct"])
+def deposit_mode(request):
+    from sputnipic_b200.device import set_plain_deposit_mode
+    prev = set_plain_deposit_mode(request.param)
+    yield request.param
+    set_plain_deposit_mode(prev)
+
+
+def launches():
+    from sputnipic_b200 import _lib
+    return _lib.load().spb_launch_count()
+
+
+@pytest.mark.parametrize("where", ["anywhere", "one cell"])
+def test_without_scratch(cuda, small_pool, deposit_mode, where):
+    """Scratch for half the particles: two chunks. None: the deposit of smaller batches, into the
+    accumulator (and its fold) or straight into the moments, as the mode says."""
+    torch = cuda
+    from sputnipic_b200 import device
+    wl = W.GemWorkload(name="t", nxc=16, nyc=8, nzc=8, Lx=4.0, Ly=2.0, Lz=2.0)
+    ctx = device.GridContext(wl)
+    for n, held, want in ((1_500_000, 0, 8),
+                          (70_001, 31 << 20, 2 if deposit_mode == "accumulator" else 1)):
+        p = particles(np.random.default_rng(n), wl, n, where)
+        d, mom = on_gpu(torch, p), torch.zeros(10, wl.nodes, device="cuda")
+        with small_pool(held):
+            before = launches()
+            ctx.p2g(d, mom)
+            assert launches() - before == want
+        assert ctx.check() == 0
+        if n < 100_000:
+            check(mom.cpu().numpy(), wl, p)
+        else:
+            whole = torch.zeros_like(mom)
+            ctx.p2g(d, whole)
+            # the same terms in runs of 16 and partial sums of other parts
+            assert float(((mom - whole).norm(dim=1) / whole.norm(dim=1)).max()) < 2e-6
+    ctx.close()
+
+
+def test_pipeline_without_scratch(cuda, small_pool, deposit_mode):
+    """interpP2G of host arrays of more than one pipeline chunk (2^22 particles), none of which gets
+    scratch: an accumulator per stream, each folded once."""
+    from sputnipic_b200 import dropin
+    dropin.release_all()
+    dropin.set_residency(False)
+    wl = W.GemWorkload(name="t", nxc=16, nyc=8, nzc=8, Lx=4.0, Ly=2.0, Lz=2.0)
+    n = (1 << 22) + 100_000
+    p = particles(np.random.default_rng(2), wl, n, "anywhere")
+    p["q"] = np.abs(p["q"])
+    p["u"], p["v"], p["w"] = (np.abs(p[k]) for k in "uvw")
+    setup = oracle.setup_from(wl)
+    ref32 = [np.zeros(wl.nodes, np.float32) for _ in range(10)]
+    oracle.CpuOracle("restated", 32).interp_p2g(setup, p, ref32)
+    ref = [np.zeros(wl.nodes) for _ in range(10)]
+    oracle.CpuOracle("restated", 64).interp_p2g(
+        setup, {k: p[k].astype(np.float64) for k in "xyzuvwq"}, ref)
+    param = dropin.make_parameters(wl)
+    grd = dropin.setGrid(param)
+    part = dropin.particle_allocate(param, 0, arrays=p)
+    ids = dropin.interp_dens_species_allocate(grd, 0)
+    with small_pool(31 << 20):
+        before = launches()
+        dropin.interpP2G(part, ids, grd, raise_on_error=True)
+        assert launches() - before == (4 if deposit_mode == "accumulator" else 2)
+    # 33,000 positive terms a node, most added one by one as the reference's FP32 code does
+    for got, r32, r in zip(dropin.moments(ids), ref32, ref):
+        err = np.linalg.norm(got.ravel() - r), np.linalg.norm(r32 - r)
+        assert err[0] <= 2 * err[1] + 1e-7 * np.linalg.norm(r)
+    dropin.release_all()
