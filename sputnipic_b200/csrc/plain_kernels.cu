@@ -670,6 +670,32 @@ __global__ void __launch_bounds__(MOVER_TPB, 7) k_plain_mover(GeomDev g, PushDev
   if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
 }
 
+// mover_interp in one pass (fused_interp says when): a warp deposits the
+// particles that it has just moved.
+template <bool ACC, bool FLOAT_CELLS, int NITER>
+__global__ void __launch_bounds__(TPB) k_plain_mover_interp(
+    GeomDev g, PushDev p, PackedFields F, float *__restrict__ x, float *__restrict__ y,
+    float *__restrict__ z, float *__restrict__ u, float *__restrict__ v,
+    float *__restrict__ w, const float *__restrict__ q, long n,
+    const __grid_constant__ DepTarget T, int *__restrict__ err) {
+  const long i = blockIdx.x * (long)TPB + threadIdx.x;
+  const bool valid = i < n;
+  Particle pt{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  int bad = 0;
+  if (valid) {
+    pt = Particle{x[i], y[i], z[i], u[i], v[i], w[i], q[i]};
+    move_one<0, FLOAT_CELLS, NITER>(g, p, F, pt.x, pt.y, pt.z, pt.u, pt.v, pt.w, bad);
+    x[i] = pt.x;
+    y[i] = pt.y;
+    z[i] = pt.z;
+    u[i] = pt.u;
+    v[i] = pt.v;
+    w[i] = pt.w;
+  }
+  deposit_warp<ACC>(g, T, valid, pt, bad);
+  if (bad) atomicOr(err, ERRBIT_OUT_OF_GRID);
+}
+
 // sumOverSpecies (src/InterpDensNet.cpp:120-146) on the device: net moment m
 // of node i = the species' values added in species order, from zero, as the
 // reference's loop does (so the float sums are bit-identical).
@@ -857,10 +883,36 @@ int launch_plain_p2g_into(const GeomDev &g, const float *x, const float *y, cons
   return SPB_OK;
 }
 
+namespace {
+// Whether mover_interp moves and deposits in one pass: below the sorted
+// deposit's threshold, where the grouped deposit takes 105 us however few the
+// particles (mover_interp of 30,000 on 64x32x32 cells: 53 us, in two passes
+// 115), and for fewer than half a particle per node, where the sorted deposit's
+// passes over the cells are its time (cell order, one pass and two: 128x64x64
+// cells, 200,000 particles 96 and 109 us, 600,000 152 and 134; 256x256x256,
+// 4M 1221 and 2000, 8M 1770 and 2313, 16M 2954 and 2835).
+bool fused_interp(const GeomDev &g, long n) {
+  return n < P2S_MIN || 2 * n < (long)g.nxn * g.nyn * g.nzn;
+}
+}  // namespace
+
 int launch_plain_mover_interp_into(const GeomDev &g, const PushDev &p, const PackedFields &F,
                                    float *x, float *y, float *z, float *u, float *v, float *w,
                                    const float *q, long n, float **acc, float *const mom[10],
                                    int *err, cudaStream_t s) {
+  if (n > 0 && fused_interp(g, n)) {
+    if (!*acc) *acc = plain_acc_alloc(g, s);
+    auto pick = [&](auto with_acc) {
+      constexpr bool A = decltype(with_acc)::value;
+      if (!g.float_cells) return k_plain_mover_interp<A, false, 0>;
+      return p.niter == 3 ? k_plain_mover_interp<A, true, 3> : k_plain_mover_interp<A, true, 0>;
+    };
+    auto *const kernel = *acc ? pick(std::true_type()) : pick(std::false_type());
+    kernel<<<blocks_for(n), TPB, 0, s>>>(g, p, F, x, y, z, u, v, w, q, n, target(*acc, mom), err);
+    SPB_CUDA(cudaGetLastError());
+    g_launches++;
+    return SPB_OK;
+  }
   if (int rc = launch_plain_mover(g, p, F, x, y, z, u, v, w, n, err, s)) return rc;
   return launch_plain_p2g_into(g, x, y, z, u, v, w, q, n, acc, mom, err, s);
 }
@@ -882,8 +934,14 @@ int launch_plain_mover_interp(const GeomDev &g, const PushDev &p, const PackedFi
                               float *x, float *y, float *z, float *u, float *v, float *w,
                               const float *q, long n, float *const mom[10], int *err,
                               cudaStream_t s) {
-  if (int rc = launch_plain_mover(g, p, F, x, y, z, u, v, w, n, err, s)) return rc;
-  return launch_plain_p2g(g, x, y, z, u, v, w, q, n, mom, err, s);
+  float *acc = nullptr;
+  const int rc =
+      launch_plain_mover_interp_into(g, p, F, x, y, z, u, v, w, q, n, &acc, mom, err, s);
+  if (rc) {
+    if (acc) cudaFreeAsync(acc, s);
+    return rc;
+  }
+  return plain_acc_fold(acc, g, mom, s);
 }
 
 int launch_apply_bc_ids(int nxn, int nyn, int nzn, const int periodic[3],

@@ -368,3 +368,32 @@ def test_pipeline_without_scratch(cuda, small_pool, deposit_mode):
         err = np.linalg.norm(got.ravel() - r), np.linalg.norm(r32 - r)
         assert err[0] <= 2 * err[1] + 1e-7 * np.linalg.norm(r)
     dropin.release_all()
+
+
+@pytest.mark.parametrize("grid,n", [((40, 24, 16), 1000), ((40, 24, 16), 65535),
+                                    ((40, 24, 16), 65536), ((64, 64, 64), 70_000),
+                                    ((64, 64, 64), 150_381), ((64, 64, 64), 150_382)])
+@pytest.mark.parametrize("where", ["anywhere", "one cell"])
+def test_mover_interp_in_one_pass_and_in_two(cuda, grid, n, where):
+    """mover_interp on both sides of its rule (65,536 particles, half a particle per node): the
+    particles that mover gives, bit for bit, and their moments."""
+    torch = cuda
+    from sputnipic_b200 import device
+    wl = W.GemWorkload(name="t", nxc=grid[0], nyc=grid[1], nzc=grid[2], Lx=grid[0] * 0.25,
+                       Ly=grid[1] * 0.25, Lz=grid[2] * 0.25, E_amp=1e-3)
+    p = particles(np.random.default_rng(n), wl, n, where)
+    one_pass = n < 65536 or 2 * n < wl.nodes
+    ctx = device.GridContext(wl)
+    ctx.set_fields(device.gen_fields(wl))
+    push = device.push_params(wl, 1)
+    moved, both = on_gpu(torch, p), on_gpu(torch, p)
+    ctx.mover(moved, push)
+    mom = torch.zeros(10, wl.nodes, device="cuda")
+    before = launches()
+    ctx.mover_interp(both, push, mom)
+    assert launches() - before == (2 if one_pass else 5)
+    assert ctx.check() == 0
+    for k in "xyzuvw":
+        assert torch.equal(moved[k], both[k])
+    check(mom.cpu().numpy(), wl, {k: v.cpu().numpy() for k, v in both.items()})
+    ctx.close()
