@@ -345,7 +345,9 @@ extern "C" int spb_grid_check(spb_grid_ctx *c, void *stream) {
   int h = 0;
   SPB_CUDA(cudaMemcpy(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (h) {
+    // cleared before the return: the next call may use another stream
     SPB_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), (cudaStream_t)stream));
+    SPB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     return fail(SPB_ERR_OUT_OF_GRID,
                 "a particle cell index left the node array; the particle was clamped to the "
                 "edge cell");

@@ -3027,6 +3027,9 @@ extern "C" int spb_sim_check(spb_sim *s, void *stream) {
   SPB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
   int h = 0;
   SPB_CUDA(cudaMemcpy(&h, s->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (h) SPB_CUDA(cudaMemsetAsync(s->d_err, 0, sizeof(int), (cudaStream_t)stream));
+  if (h) {   // cleared before the return: the next call may use another stream
+    SPB_CUDA(cudaMemsetAsync(s->d_err, 0, sizeof(int), (cudaStream_t)stream));
+    SPB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  }
   return spb::sim_status(h);
 }

@@ -78,3 +78,27 @@ def test_moments_written_right_after_creation(cuda):
     torch.cuda.synchronize()
     assert torch.equal(sim.moments_view(0).view_as(want), want)
     sim.close()
+
+
+def test_reported_errors_are_cleared_for_every_stream(cuda):
+    """check() clears the error word before it returns: a particle off the grid that another stream
+    deposits right after it is reported, and a clean deposit then is not."""
+    torch = cuda
+    from sputnipic_b200 import _lib, device
+
+    wl = W.small_gem(nxc=16, nyc=8, nzc=8, species=W.gem_species((8, 8, 8, 8)))
+    bad = device.gen_particles(wl, 0)
+    good = {k: v.clone() for k, v in bad.items()}
+    bad["y"][7] = 1e9
+    mom = torch.zeros(10, wl.nodes, device="cuda")
+    torch.cuda.synchronize()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    ctx = device.GridContext(wl)
+    for _ in range(20):
+        for st in (a, b):
+            ctx.p2g(bad, mom, stream=st)
+            with pytest.raises(_lib.SpbError):
+                _lib.check(ctx.check(st))
+    ctx.p2g(good, mom, stream=a)
+    assert ctx.check(a) == 0
+    ctx.close()
