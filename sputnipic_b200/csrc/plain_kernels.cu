@@ -469,7 +469,7 @@ __device__ __forceinline__ void deposit_lone(const GeomDev &g, const DepTarget &
 // 80 adds serve the whole group instead of one per 32 particles. Groups of up
 // to three particles deposit particle by particle (deposit_lone). A chunk
 // with more distinct cells than the table holds (unordered input) deposits
-// every particle by itself (deposit_lone).
+// warp by warp (deposit_warp).
 constexpr int GP_TPB = 256;
 constexpr int GP_PER_THREAD = 4;
 constexpr int GP_CHUNK = GP_TPB * GP_PER_THREAD;
@@ -490,8 +490,8 @@ __device__ __forceinline__ Particle smem_particle(const GroupSmem &S, int j) {
   return Particle{S.p[0][j], S.p[1][j], S.p[2][j], S.p[3][j], S.p[4][j], S.p[5][j], S.p[6][j]};
 }
 
-// (Particles in the arrays' own order: deposits below P2S_MIN particles and
-// those whose scratch cannot be had; the others go through sorted_p2g.)
+// (Particles in the arrays' own order: interpP2G below P2S_MIN particles, and
+// deposits whose scratch for the cell order cannot be had.)
 template <bool ACC>
 __global__ void __launch_bounds__(GP_TPB) k_plain_p2g_grouped(
     GeomDev g, const float *__restrict__ x, const float *__restrict__ y,

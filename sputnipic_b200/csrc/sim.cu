@@ -512,6 +512,13 @@ struct PushWarp {
   int bad = 0, lost = 0;
 };
 
+// Whether a destination tile coordinate d tiles away on an axis of n tiles
+// (periodic or not) lies outside the source tile's neighbourhood.
+__device__ __forceinline__ bool far_axis(int d, int n, int periodic) {
+  if (periodic && n > 2) d = d == n - 1 ? -1 : (d == 1 - n ? 1 : d);
+  return d < -1 || d > 1;
+}
+
 // Species [s0, s1) of one tile (tile-local index `tile` of the job P) on the
 // staged fields sF. All threads call.
 //
@@ -525,13 +532,6 @@ struct PushWarp {
 // of their own per cell, waits, and 24 of the 160 passes through the shared-
 // memory pipe per slot. GEM grid, 4 species: 7021 -> 6239 us at 125 particles per
 // cell, 1735 -> 1479 us at 27, 691 -> 532 us at 8.
-// Whether a destination tile coordinate d tiles away on an axis of n tiles
-// (periodic or not) lies outside the source tile's neighbourhood.
-__device__ __forceinline__ bool far_axis(int d, int n, int periodic) {
-  if (periodic && n > 2) d = d == n - 1 ? -1 : (d == 1 - n ? 1 : d);
-  return d < -1 || d > 1;
-}
-
 template <int TX, int TY, int TZ, bool FUSED = false>
 __device__ __forceinline__ void push_tile(const CycleParams &P, int tile, int s0, int s1,
                                           const float *sF, PushWarp &W) {
@@ -1420,9 +1420,7 @@ __global__ void __launch_bounds__(SIM_TPB, MINB)
         return;
       }
       deposit_tile<TX, TY, TZ, SIM_TPB, true>(P, tile, 0, P.ns, sCell);
-      // the next tile's bulk copies overwrite the sums written here
-      fence_proxy_async();
-      __syncthreads();
+      __syncthreads();   // the next tile's staged records overwrite the sums
     }
   }
   report(P, W);
@@ -1819,8 +1817,8 @@ cudaError_t dmalloc(T **p, size_t bytes) {
   cudaStream_t st = pool_stream();
   cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(p), std::max<size_t>(bytes, 1), st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  // the kernels move records with 32-byte accesses and bulk copies: every
-  // array must start on (at least) a 256-byte boundary, as device
+  // the kernels move records with 32-byte accesses and the fields with tensor
+  // copies: every array must start on (at least) a 256-byte boundary, as device
   // allocations do
   if (e == cudaSuccess && (reinterpret_cast<uintptr_t>(*p) & 255u)) {
     cudaFreeAsync(*p, st);
@@ -1866,7 +1864,7 @@ int encode_field_map(spb_sim *s) {
 
 // Dynamic shared memory of the kernels; the multi-job kernels also stage one
 // job's parameters.
-template <int TX, int TY, int TZ, int MINB>
+template <int TX, int TY, int TZ>
 size_t push_smem(bool multi = false) {
   return 2 * (size_t)Tile<TX, TY, TZ>::SF * 4 + (size_t)SIM_NW * 64 * sizeof(float4) +
          (multi ? sizeof(CycleParams) : 0) + 2 * sizeof(uint64_t);
@@ -1948,7 +1946,7 @@ int launch_cycle_v(spb_sim *s, cudaStream_t st) {
   k_zero_cycle<<<blocks_for(5 * s->nodes, 256), 256, 0, st>>>(P);
   SPB_CUDA(cudaGetLastError());
   const bool exact = s->d.deterministic != 0;
-  const size_t psm = push_smem<TX, TY, TZ, MINB>(), dsm = deposit_smem<TX, TY, TZ>(false, exact);
+  const size_t psm = push_smem<TX, TY, TZ>(), dsm = deposit_smem<TX, TY, TZ>(false, exact);
   auto *const kdep = exact ? k_deposit<TX, TY, TZ, false, true> : k_deposit<TX, TY, TZ, false, false>;
   static bool attr = false;
   if (!attr) {
@@ -2351,7 +2349,7 @@ int ensure_job_buffers(JobBuffers &B, int n) {
 template <int TX, int TY, int TZ>
 int launch_jobs_t(spb_sim *const *sims, int n, JobBuffers &B, cudaStream_t st) {
   constexpr int MINB = 3;
-  const size_t psm = push_smem<TX, TY, TZ, MINB>(true), dsm = deposit_smem<TX, TY, TZ>(true);
+  const size_t psm = push_smem<TX, TY, TZ>(true), dsm = deposit_smem<TX, TY, TZ>(true);
   static int pocc = 0, docc = 0;
   if (!pocc) {
     SPB_CUDA(cudaFuncSetAttribute(k_push<TX, TY, TZ, MINB, true>,
