@@ -302,7 +302,7 @@ bool share(const T *a, long na, const T *b, long nb) {
 }
 
 int blocks_for(long n, int tpb) {
-  return (int)std::max<long>(1, std::min<long>((n + tpb - 1) / tpb, 148L * 16));
+  return (int)std::max<long>(1, std::min<long>((n + tpb - 1) / tpb, 16L * num_sms()));
 }
 
 template <typename T>
@@ -346,7 +346,7 @@ int hat_densities(const spb_hat_desc *d, const T *const *mom, const T *const B[3
   int rc = SPB_OK;
   // cells per thread along x: eight, fewer where that would leave SMs without
   // a full set of threads
-  const int run = (int)std::max(1L, std::min(8L, inner * ns / (148L * 512)));
+  const int run = (int)std::max(1L, std::min(8L, inner * ns / (512L * num_sms())));
   const dim3 grid((unsigned)(ceil_div((long)(g.nyc - 2) * (g.nzc - 2), 128) *
                              ceil_div(g.nxc - 2, run)), (unsigned)ns);
   k_hat_div_tensor<T><<<grid, 128, 0, st>>>(g, S, alfa, run);

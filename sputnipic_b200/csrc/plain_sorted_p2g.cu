@@ -459,7 +459,7 @@ int sorted_p2g_by(const GeomDev &g, const float *x, const float *y, const float 
   int rc = SPB_OK;
   for (long off = 0; off < n && rc == SPB_OK; off += chunk) {
     const long c = std::min(chunk, n - off);
-    const unsigned blocks = (unsigned)std::min<long>(ceil_div(c, TPB), 148L * 32);
+    const unsigned blocks = (unsigned)std::min<long>(ceil_div(c, TPB), 32L * num_sms());
     const Particles7 P{{x + off, y + off, z + off, u + off, v + off, w + off, q + off}};
     cudaError_t e = cudaMemsetAsync(count, 0, (size_t)(keys + 2) * sizeof(unsigned), s);
     if (e == cudaSuccess) {
