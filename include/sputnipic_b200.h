@@ -71,11 +71,13 @@ const char *spb_version(void);
 /* Number of kernels this library has launched in this process. */
 long spb_launch_count(void);
 
-/* How the plain interpP2G / mover_interp deposits (process-wide):
- * it concerns deposits of fewer than 65,536 particles and those that cannot
- * get the scratch of the sorted deposit (32 bytes per particle of a chunk of
- * at most 2^26 particles, halved until it can be had, from the device's
- * stream-ordered pool), which adds straight into the ten arrays.
+/* How the plain interpP2G / mover_interp deposits where it does not go through
+ * particles in cell order (process-wide): interpP2G of fewer than 65,536
+ * particles, mover_interp of those or of fewer than half a particle per node,
+ * and deposits that cannot get the cell order's scratch (32 bytes per particle
+ * of a chunk of at most 2^26 particles, halved until it can be had, from the
+ * device's stream-ordered pool). The deposit in cell order adds straight into
+ * the ten arrays in either mode.
  * SPB_DEPOSIT_ACCUMULATOR (default) adds into a node-interleaved buffer of
  * 48 bytes per node from the pool, then into the ten moment arrays (fewer L2
  * transactions); SPB_DEPOSIT_DIRECT adds straight into the ten arrays. The
@@ -154,8 +156,9 @@ int spb_particle_sort(struct parameters *param, struct particles *part, struct g
  * interpP2G moment order; entries 1..9 are read), B the three magnetic
  * field node arrays, rhoc the centre array [nxc][nyc][nzc] (guards
  * included); outputs as the drop-in's. An output may be an input array: J hat
- * any of the moments or B, rho hat rhoc, a moment or B. Asynchronous on
- * `stream`. */
+ * any of the moments or B, rho hat rhoc, a moment or B. Scratch (3 ns centre
+ * arrays) comes from the device's stream-ordered pool, whose freed memory the
+ * library keeps until spb_release_cached_memory. Asynchronous on `stream`. */
 struct interpDens_aux;
 #define SPB_HAT_MAX_SPECIES 16
 typedef struct spb_hat_desc {
@@ -234,7 +237,8 @@ int spb_grid_mover(spb_grid_ctx *ctx, const spb_push *push, float *x, float *y,
 int spb_grid_p2g(spb_grid_ctx *ctx, const float *x, const float *y,
                  const float *z, const float *u, const float *v, const float *w,
                  const float *q, long n, float *const mom[10], void *stream);
-/* mover_interp: spb_grid_mover, then spb_grid_p2g on the moved particles. */
+/* mover_interp: spb_grid_mover, then spb_grid_p2g on the moved particles (in
+ * one pass below 65,536 particles or half a particle per node). */
 int spb_grid_mover_interp(spb_grid_ctx *ctx, const spb_push *push, float *x,
                           float *y, float *z, float *u, float *v, float *w,
                           const float *q, long n, float *const mom[10],

@@ -41,8 +41,9 @@ DEPOSIT_MODES = {"accumulator": 0, "direct": 1}
 
 
 def set_plain_deposit_mode(mode: str) -> str:
-    """How the plain interpP2G / mover_interp deposits where it does not sort
-    (fewer than 65,536 particles, or no scratch for the sorted deposit),
+    """How the plain interpP2G / mover_interp deposits where it does not go through
+    particles in cell order (fewer than 65,536 particles, for mover_interp also
+    fewer than half a particle per node, or no scratch for the cell order),
     process-wide (spb_set_plain_deposit_mode): "accumulator" (a
     node-interleaved buffer from the device pool, then added into the ten
     moment arrays; the default) or "direct" (straight into the ten arrays).
