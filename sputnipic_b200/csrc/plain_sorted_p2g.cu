@@ -456,6 +456,8 @@ int sorted_p2g_by(const GeomDev &g, const float *x, const float *y, const float 
   const Heavy H{(unsigned)std::max<long>(HEAVY_MIN, chunk / (inner * (TC / 8))),
                 (unsigned)std::max(2L * HEAVY_MIN, ceil_div(chunk, (long)places * (TC / 32))),
                 segs};
+  // a warp for every segment that there can be, no more CTAs than fit
+  const int seg_ctas = (int)std::min<long>(places, ceil_div(chunk / HEAVY_MIN, TC / 32));
   int rc = SPB_OK;
   for (long off = 0; off < n && rc == SPB_OK; off += chunk) {
     const long c = std::min(chunk, n - off);
@@ -471,7 +473,7 @@ int sorted_p2g_by(const GeomDev &g, const float *x, const float *y, const float 
       k_p2g_bases<<<(unsigned)ceil_div(keys, BASES_TPB), BASES_TPB, 0, s>>>(count, keys, next,
                                                                             taken, H);
       k_records<<<blocks, TPB, 0, s>>>(g, nty, ntz, P, c, next, rec, err);
-      k_p2g_cells<TX, TY, TZ><<<(unsigned)(tiles * parts + places), TC, 0, s>>>(
+      k_p2g_cells<TX, TY, TZ><<<(unsigned)(tiles * parts + seg_ctas), TC, 0, s>>>(
           g, nty, ntz, (int)tiles, parts, count, next, taken + 1, H, rec, M);
       e = cudaGetLastError();
     }
