@@ -139,7 +139,7 @@ __device__ __forceinline__ double d4_planes(const HatGeom &g, const Plane6<T> &l
 // a cell costs 24 loads (four nodes of six components) instead of the 72 that
 // its nine stencils read one by one: those kept the L1 pipe busy (an unaligned
 // row of 32 doubles takes three passes). 128x64x64 cells, 4 species, FP64: 62 ->
-// 46 us; with the guard fills gone the whole call 168 -> 110 us. Register caps
+// 46 us; with the guard fills gone the whole call 168 -> 106 us. Register caps
 // for four (double) and five (float) CTAs per SM: float 83 -> 74 us.
 template <typename T>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 5) k_hat_div_tensor(HatGeom g, const __grid_constant__ Species6<T> S, T alfa, int run) {

@@ -14,8 +14,8 @@
 // deposit 4-byte gathers through it, 4.5 L2 sectors per particle in arrays
 // near cell order and up to 7 in others, and a warp reduction per run of a
 // cell's particles. 65.5M particles in cell order, 125 per cell, zeroing and
-// applyBCids included: 2352 -> 1455 us (count 150, copy 680, sum 600); two
-// species of 2.4M some cycles after the last sort, 27 per cell: 432 -> 232 us.
+// applyBCids included: 2376 -> 1468 us (count 150, copy 680, sum 610); two
+// species of 2.4M some cycles after the last sort, 27 per cell: 433 -> 231 us.
 //
 // Cells are numbered tile by tile (8 x 4 x 4 cells, on thin grids of one layer;
 // a CTA of the last launch takes a tile), over the nxn - 1 cells per axis that
