@@ -197,7 +197,7 @@ __device__ __forceinline__ void add_record(float2 (&acc)[40], const CellNodes &N
 // The heavy cells' segments, one per warp at a time: neighbouring lanes take
 // neighbouring records, and every SUM_RUN of a lane's are summed over the warp
 // into doubles (in shared memory, five per thread: the sums at hand fill the
-// registers).
+// registers; a record loaded ahead spilled and gained nothing).
 template <int TX, int TY, int TZ>
 __device__ __forceinline__ void sum_segments(const GeomDev &g, int nty, int ntz, int cta, int ctas,
                                              const unsigned *__restrict__ nsegs,
@@ -218,8 +218,6 @@ __device__ __forceinline__ void sum_segments(const GeomDev &g, int nty, int ntz,
     double *const sum = sums + threadIdx.x;
 #pragma unroll
     for (int k = 0; k < 5; ++k) sum[k * TC] = 0.0;
-    float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na;
-    if (lane < seg.y) ld_rec(rec + 2 * lane, na, nb);
 #pragma unroll 1
     for (int o = 0; o < seg.y;) {
       float2 acc[40];
@@ -227,10 +225,12 @@ __device__ __forceinline__ void sum_segments(const GeomDev &g, int nty, int ntz,
       for (int i = 0; i < 40; ++i) acc[i] = make_float2(0.f, 0.f);
       const int stop = min(o + 32 * SUM_RUN, seg.y);
 #pragma unroll 1
-      for (; o < stop; o += 32) {
-        float4 a,b; if (o + lane < seg.y) ld_rec(rec + 2 * (o + lane), a, b);
-        if (o + lane < seg.y) add_record(acc, N, inv, a, b, lane);
-      }
+      for (; o < stop; o += 32)
+        if (o + lane < seg.y) {
+          float4 a, b;
+          ld_rec(rec + 2 * (o + lane), a, b);
+          add_record(acc, N, inv, a, b, lane);
+        }
       float r[5];
       warp_sum80(acc, r, lane);
 #pragma unroll
@@ -273,10 +273,10 @@ __device__ __forceinline__ void add_cell(const GeomDev &g, const CellNodes &N, i
 
 // The first CTAs take one tile of cells and one of `parts` parts of each cell's
 // records, the last ones the heavy cells' segments (none on most input: they
-// end as the last tiles are summed). Thread t sums the records of cell t, the warp those above its
-// quota (deposit_quota), and every node of the tile adds its cells' sums into
-// the moments. A term is f (q xi) eta (zeta invVOL),
-// summed in FP32; the second invVOL multiplies a node's sum once (the reference
+// end as the last tiles are summed). Thread t sums the records of cell t, the
+// warp those above its quota (deposit_quota), and every node of the tile adds
+// its cells' sums into the moments. A term is f (q xi) eta (zeta invVOL), summed
+// in FP32; the second invVOL multiplies a node's sum once (the reference
 // multiplies every term by both): fewer roundings than its own. (q invVOL
 // would round alike for all particles of equal charge: a bias, not noise.)
 template <int TX, int TY, int TZ>
@@ -409,9 +409,9 @@ long inner_tiles(const GeomDev &g) {
 }
 
 template <int TX, int TY, int TZ>
-int sorted_p2g_by(const GeomDev &g, const float *x, const float *y, const float *z, const float *u,
-               const float *v, const float *w, const float *q, long n, float *const mom[10],
-               int *err, cudaStream_t s, long *done) {
+int sorted_p2g_by(const GeomDev &g, const float *x, const float *y, const float *z,
+                  const float *u, const float *v, const float *w, const float *q, long n,
+                  float *const mom[10], int *err, cudaStream_t s, long *done) {
   *done = 0;
   const int ntx = (int)ceil_div(g.nxn + TX - 2, TX), nty = (int)ceil_div(g.nyn + TY - 2, TY),
             ntz = (int)ceil_div(g.nzn + TZ - 2, TZ);
